@@ -54,7 +54,7 @@ struct DevBricks {
 template <bool kStats>
 __device__ Info scene_distance_skip(const DevScene& S, F3 p, const DevBricks& B, Ctx<kStats>& cx) {
   float best = kInf;
-  Info cur{kInf, 0u, 0u};
+  Info cur{kInf, ftd::kNoRef};
   int stack[64];
   float stack_lb[64];
   int sp = 0;
@@ -173,7 +173,7 @@ struct BrickBuild {
 };
 
 // Sample the cached field at every lattice point.
-__global__ void __launch_bounds__(128) brick_lattice_kernel(DevScene S, DevBricks B, BrickBuild G,
+__global__ void __launch_bounds__(128) brick_lattice_kernel(const __grid_constant__ DevScene S, const __grid_constant__ DevBricks B, BrickBuild G,
                                                             float* __restrict__ lattice) {
   Ctx<false> cx;
   cx.c = Counters{};
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256) brick_texel_kernel(BrickBuild G, const fl
 }
 
 // Validation: the far-field bound and the exact distance at given points.
-__global__ void brick_query_kernel(DevScene S, DevBricks B, const float* __restrict__ pts, uint32_t n,
+__global__ void brick_query_kernel(const __grid_constant__ DevScene S, const __grid_constant__ DevBricks B, const float* __restrict__ pts, uint32_t n,
                                    float* __restrict__ bound, float* __restrict__ exact) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;

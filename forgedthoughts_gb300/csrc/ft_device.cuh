@@ -33,6 +33,17 @@ FT_DEV F3 normalize3(F3 a) {
   return a * (1.0f / l);
 }
 
+// normalize3 with its multiply-adds written out, the squares summed x or y
+// first (an ulp of a primary ray moves a silhouette pixel, so each kernel
+// keeps its order whatever the compiler contracts).
+template <bool kYFirst>
+FT_DEV F3 normalize3_fma(F3 a) {
+  const float u = kYFirst ? a.y : a.x, v = kYFirst ? a.x : a.y;
+  const float l = sqrtf(fmaf(a.z, a.z, fmaf(u, u, v * v)));
+  if (l <= 1.1920929e-7f) return a;
+  return a * (1.0f / l);
+}
+
 // Rust f32::max / f32::min / f32::clamp.
 FT_DEV float rmax(float a, float b) { return fmaxf(a, b); }
 FT_DEV float rmin(float a, float b) { return fminf(a, b); }
@@ -46,10 +57,16 @@ FT_DEV float rem_euclid(float a, float b) {
   return r < 0.0f ? r + fabsf(b) : r;
 }
 
-struct Info {  // DistanceInfo (R:454-459)
+// DistanceInfo (R:454-459).  The object and material ids of the nearest
+// surface are those of one primitive, so an evaluation carries a reference to
+// it (half the registers of the two ids) and the ids are read where a hit is
+// recorded: a node index, the complement of a compact primitive's index
+// (negative), or kNoRef.
+struct Info {
   float d;
-  uint32_t obj, mat;
+  int32_t ref;
 };
+constexpr int32_t kNoRef = 0x7fffffff;
 
 // Scene node as laid out in device memory: the IR node plus the sin/cos of
 // the inverse rotation angles, computed once on the host with the same f32
@@ -71,7 +88,7 @@ FT_DEV F3 to_local(F3 p, const DevNode& n) {
   F3 q = f3(p.x - n.c[0], p.y - n.c[1], p.z - n.c[2]);
   if (!n.has_rot) return q;
   q = f3(n.cz * q.x - n.sz * q.y, n.sz * q.x + n.cz * q.y, q.z);
-  q = f3(n.cy * q.x + n.sy * q.z, q.y, -n.sy * q.x + n.cy * q.z);
+  q = f3(fmaf(n.cy, q.x, n.sy * q.z), q.y, fmaf(n.cy, q.z, -n.sy * q.x));
   q = f3(q.x, n.cx * q.y - n.sx * q.z, n.sx * q.y + n.cx * q.z);
   return q;
 }
@@ -93,36 +110,32 @@ __device__ __noinline__ float sd_regular_ngon(float px, float pz, int sides, flo
 
 __device__ __noinline__ float prim_local_rare(int kind, const float* f, int ival, F3 q);
 
-// Primitive arms of sdf_distance_info (R:5547-5663), point already local.
+// Sphere and box arms of sdf_distance_info (R:5547-5663), point already local.
+// Multiply-adds written out, as in compact_distance.
+FT_DEV float sphere_local(const float* f, F3 q) {
+  return shell(sqrtf(fmaf(q.z, q.z, fmaf(q.y, q.y, q.x * q.x))) - f[0], f[1]);
+}
+FT_DEV float box_local(const float* f, F3 q) {
+  const float rd = f[3];
+  const float ix = rmax(f[0] - rd, 0.0f), iy = rmax(f[1] - rd, 0.0f), iz = rmax(f[2] - rd, 0.0f);
+  const float qx = fabsf(q.x) - ix, qy = fabsf(q.y) - iy, qz = fabsf(q.z) - iz;
+  const float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
+  const float outside = sqrtf(fmaf(oz, oz, fmaf(ox, ox, oy * oy)));
+  const float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);
+  return shell(outside + inside - rd, f[4]);
+}
+
 // Spheres and boxes inline; the other kinds out of line.
 FT_DEV float prim_local(int kind, const float* f, int ival, F3 q) {
   switch (kind) {
-    case FT_NODE_SPHERE: return shell(len3(q) - f[0], f[1]);
-    case FT_NODE_BOX: {
-      float rd = f[3];
-      float ix = rmax(f[0] - rd, 0.0f), iy = rmax(f[1] - rd, 0.0f), iz = rmax(f[2] - rd, 0.0f);
-      float qx = fabsf(q.x) - ix, qy = fabsf(q.y) - iy, qz = fabsf(q.z) - iz;
-      float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
-      float outside = sqrtf(ox * ox + oy * oy + oz * oz);
-      float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);
-      return shell(outside + inside - rd, f[4]);
-    }
+    case FT_NODE_SPHERE: return sphere_local(f, q);
+    case FT_NODE_BOX: return box_local(f, q);
     default: return prim_local_rare(kind, f, ival, q);
   }
 }
 
 __device__ __noinline__ float prim_local_rare(int kind, const float* f, int ival, F3 q) {
   switch (kind) {
-    case FT_NODE_SPHERE: return shell(len3(q) - f[0], f[1]);
-    case FT_NODE_BOX: {
-      float rd = f[3];
-      float ix = rmax(f[0] - rd, 0.0f), iy = rmax(f[1] - rd, 0.0f), iz = rmax(f[2] - rd, 0.0f);
-      float qx = fabsf(q.x) - ix, qy = fabsf(q.y) - iy, qz = fabsf(q.z) - iz;
-      float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
-      float outside = sqrtf(ox * ox + oy * oy + oz * oz);
-      float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);
-      return shell(outside + inside - rd, f[4]);
-    }
     case FT_NODE_CYLINDER: {
       float rd = f[2];
       float radial = sqrtf(q.x * q.x + q.z * q.z);
@@ -152,6 +165,30 @@ __device__ __noinline__ float prim_local_rare(int kind, const float* f, int ival
 
 FT_DEV float prim_distance(const DevNode& n, F3 p) { return prim_local(n.kind, n.f, n.ival, to_local(p, n)); }
 
+// Compact primitive: a sphere, or a box with or without rounding, turned about
+// y at most, as three 16-byte words
+//   { centre, cos }, { h, rd }, { sin, shell, node, leaf | rare flag }
+// with the sin / cos of DevNode, h the box's half size less its rounding rd
+// (0 and the radius for a sphere, whose distance is that of a box of no size
+// rounded by the radius) and shell = +inf where there is none.  One branch-free
+// formula in 48 bytes serves every lane; each term is the one prim_local
+// computes (the sphere's |q| - 0, the unturned box's 1 q.x + 0 q.z and the
+// absent shell's max(d, -inf) are exact).  The multiply-adds are written out:
+// every kernel rounds a distance alike, whatever the compiler contracts around
+// it, so that the depth march and the wavefront march take the same steps.
+// Other kinds set the rare flag and go through their node.
+constexpr uint32_t kRareFlag = 0x80000000u;
+FT_DEV float compact_distance(float4 a, float4 b, float sn, float sh, F3 p) {
+  const F3 t = f3(p.x - a.x, p.y - a.y, p.z - a.z);
+  const float qx = fabsf(fmaf(a.w, t.x, sn * t.z)) - b.x, qy = fabsf(t.y) - b.y,
+              qz = fabsf(fmaf(a.w, t.z, -sn * t.x)) - b.z;
+  const float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
+  const float outside = sqrtf(fmaf(oz, oz, fmaf(ox, ox, oy * oy)));
+  const float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);
+  const float d = outside + inside - b.w;
+  return rmax(d, -(d + sh));
+}
+
 // Device-wide nanosecond timer (%globaltimer), for time limits of long loops.
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -159,13 +196,14 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// point_aabb_lower_bound (R:5388-5411)
-FT_DEV float aabb_lb(F3 p, const float* mn, const float* mx) {
+// point_aabb_lower_bound (R:5388-5411), and its square
+FT_DEV float aabb_lb2(F3 p, const float* mn, const float* mx) {
   float dx = p.x < mn[0] ? mn[0] - p.x : (p.x > mx[0] ? p.x - mx[0] : 0.0f);
   float dy = p.y < mn[1] ? mn[1] - p.y : (p.y > mx[1] ? p.y - mx[1] : 0.0f);
   float dz = p.z < mn[2] ? mn[2] - p.z : (p.z > mx[2] ? p.z - mx[2] : 0.0f);
-  return sqrtf(dx * dx + dy * dy + dz * dz);
+  return dx * dx + dy * dy + dz * dz;
 }
+FT_DEV float aabb_lb(F3 p, const float* mn, const float* mx) { return sqrtf(aabb_lb2(p, mn, mx)); }
 
 // ---------------------------------------------------------- hg_sdf operators
 constexpr float kFrac1Sqrt2 = 0.70710678118654752440f;
@@ -173,7 +211,7 @@ constexpr float kFrac1Sqrt2 = 0.70710678118654752440f;
 FT_DEV float op_union_round(float a, float b, float r) {
   r = rmax(fabsf(r), 1.0e-6f);
   float ux = rmax(r - a, 0.0f), uy = rmax(r - b, 0.0f);
-  return rmax(r, rmin(a, b)) - sqrtf(ux * ux + uy * uy);
+  return rmax(r, rmin(a, b)) - sqrtf(fmaf(ux, ux, uy * uy));
 }
 FT_DEV float op_intersect_round(float a, float b, float r) {
   r = rmax(fabsf(r), 1.0e-6f);
@@ -234,7 +272,7 @@ FT_DEV Info combine(int kind, float ra, float rb, Info l, Info r) {
     case FT_NODE_SUBTRACT: {
       float rd = -r.d;
       if (l.d >= rd) return l;
-      return Info{rd, r.obj, r.mat};
+      return Info{rd, r.ref};
     }
     case FT_NODE_UNION_ROUND: d = op_union_round(l.d, r.d, ra); break;
     case FT_NODE_UNION_CHAMFER: d = op_union_chamfer(l.d, r.d, ra); break;
@@ -249,15 +287,15 @@ FT_DEV Info combine(int kind, float ra, float rb, Info l, Info r) {
     case FT_NODE_DIFF_CHAMFER: d = op_intersect_chamfer(l.d, -r.d, ra); break;
     case FT_NODE_DIFF_COLUMNS: d = -op_union_columns(-l.d, r.d, ra, rb); break;
     case FT_NODE_DIFF_STAIRS: d = -op_union_stairs(-l.d, r.d, ra, rb); break;
-    case FT_NODE_PIPE: return Info{sqrtf(l.d * l.d + r.d * r.d) - fabsf(ra), l.obj, l.mat};
-    case FT_NODE_ENGRAVE: return Info{rmax(l.d, (l.d + fabsf(ra) - fabsf(r.d)) * kFrac1Sqrt2), l.obj, l.mat};
-    case FT_NODE_GROOVE: return Info{rmax(l.d, rmin(l.d + fabsf(ra), fabsf(rb) - fabsf(r.d))), l.obj, l.mat};
-    case FT_NODE_TONGUE: return Info{rmin(l.d, rmax(l.d - fabsf(ra), fabsf(r.d) - fabsf(rb))), l.obj, l.mat};
+    case FT_NODE_PIPE: return Info{sqrtf(l.d * l.d + r.d * r.d) - fabsf(ra), l.ref};
+    case FT_NODE_ENGRAVE: return Info{rmax(l.d, (l.d + fabsf(ra) - fabsf(r.d)) * kFrac1Sqrt2), l.ref};
+    case FT_NODE_GROOVE: return Info{rmax(l.d, rmin(l.d + fabsf(ra), fabsf(rb) - fabsf(r.d))), l.ref};
+    case FT_NODE_TONGUE: return Info{rmin(l.d, rmax(l.d - fabsf(ra), fabsf(r.d) - fabsf(rb))), l.ref};
     default: return l;
   }
-  if (kind <= FT_NODE_UNION_SOFT) return l.d <= r.d ? Info{d, l.obj, l.mat} : Info{d, r.obj, r.mat};
-  if (kind <= FT_NODE_INTERSECT_STAIRS) return l.d >= r.d ? Info{d, l.obj, l.mat} : Info{d, r.obj, r.mat};
-  return l.d >= -r.d ? Info{d, l.obj, l.mat} : Info{d, r.obj, r.mat};
+  if (kind <= FT_NODE_UNION_SOFT) return l.d <= r.d ? Info{d, l.ref} : Info{d, r.ref};
+  if (kind <= FT_NODE_INTERSECT_STAIRS) return l.d >= r.d ? Info{d, l.ref} : Info{d, r.ref};
+  return l.d >= -r.d ? Info{d, l.ref} : Info{d, r.ref};
 }
 
 // ---------------------------------------------------------- noise (R:5957-6017)

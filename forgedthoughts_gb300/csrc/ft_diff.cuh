@@ -279,7 +279,7 @@ __device__ bool scene_backprop(const DevScene& S, F3 p, float* vals, float* adjs
 }
 
 // One thread per (view, work item).
-__global__ void __launch_bounds__(128) views_forward_kernel(DevScene S, const RayParams* __restrict__ views,
+__global__ void __launch_bounds__(128) views_forward_kernel(const __grid_constant__ DevScene S, const RayParams* __restrict__ views,
                                                             uint32_t n_views, uint64_t items_per_view, float tau,
                                                             float* __restrict__ t_out, uint8_t* __restrict__ mask_out,
                                                             float* __restrict__ sil_out) {
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(128) views_forward_kernel(DevScene S, const Ra
 
 // Adjoint: recompute each ray, then accumulate its parameter gradient.
 // Dynamic shared memory: n_params doubles when `shared_acc`.
-__global__ void __launch_bounds__(128) views_backward_kernel(DevScene S, const RayParams* __restrict__ views,
+__global__ void __launch_bounds__(128) views_backward_kernel(const __grid_constant__ DevScene S, const RayParams* __restrict__ views,
                                                              uint32_t n_views, uint64_t items_per_view, float tau,
                                                              DiffTables T, const float* __restrict__ dl_dt,
                                                              const float* __restrict__ dl_dsil, double* __restrict__ grad,
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(128) views_backward_kernel(DevScene S, const R
     const RayParams& P = views[v];
     F3 d;
     size_t idx = 0;
-    if (!item_ray(P, g - static_cast<uint64_t>(v) * items_per_view, &d, &idx)) continue;
+    if (!item_ray<true>(P, g - static_cast<uint64_t>(v) * items_per_view, &d, &idx)) continue;
     idx += static_cast<size_t>(v) * P.width * P.height;
     float wt = dl_dt ? dl_dt[idx] : 0.0f, ws = dl_dsil ? dl_dsil[idx] : 0.0f;
     if (wt == 0.0f && ws == 0.0f) continue;

@@ -35,17 +35,19 @@ struct DevBvhNode {
   float bmin[3], bmax[3];
   int32_t lhs, rhs, leaf, pad;
 };
+// Candidate grid: cell c of the box from gmin lists (DevScene::cells, cell
+// first + c) the primitives that can be the nearest or lie within the blend
+// radius at some point of it.  dims[0] == 0: none.
+struct DevGrid {
+  float gmin[3];
+  float inv_cell;
+  int32_t dims[3];
+  int32_t first;
+};
 struct DevUrTree {
   float r;
   int32_t n_prims, prim_first, bvh_root, inner_root, depth, fallback_first, fallback_count;
-  float gmin[3];
-  float cell, inv_cell;
-  int32_t dims[3];
-  int32_t cell_first, pad;
-  float ogmin[3];
-  float ocell, oinv_cell;
-  int32_t odims[3];
-  int32_t ocell_first, opad;
+  DevGrid fine, outer;
 };
 struct DevUrBvh {
   float bmin[3], bmax[3];
@@ -56,7 +58,22 @@ struct DevUrInner {
   int32_t lo, hi;
 };
 
+// Scenes whose distance has a short form, taken by the march loops without
+// the general leaf walk.  kFastTree: one union_round tree, alone or beside one
+// primitive (a ground); the copies of the tree's header and the leaf boxes are
+// kernel parameters, read from the constant bank.
+enum FastKind : int32_t { kFastNone = 0, kFastTree = 1 };
+struct DevFast {
+  int32_t kind;
+  uint32_t prim;       // kFastTree: the primitive leaf's compact entry, kNoPrim for a tree alone
+  int32_t tree_lhs;    // the tree is the BVH root's left child
+  float pmin[3], pmax[3], tmin[3], tmax[3];
+  DevUrTree tree;
+};
+constexpr uint32_t kNoPrim = 0xffffffffu;
+
 struct DevScene {
+  DevFast fast;
   const DevNode* __restrict__ nodes;
   const DevLeaf* __restrict__ leaves;
   const DevBvhNode* __restrict__ bvh;
@@ -66,8 +83,10 @@ struct DevScene {
   const int32_t* __restrict__ ur_bvh_prims;
   const int32_t* __restrict__ ur_prims;
   const DevUrInner* __restrict__ ur_inner;
-  const uint32_t* __restrict__ ur_cell_offsets;
-  const int32_t* __restrict__ ur_cell_prims;
+  const float4* __restrict__ cprims;   // compact primitives (three words each, compact_distance)
+  const uint4* __restrict__ ur_paths;  // per tree primitive: sides taken from the root (low, high word), depth
+  const uint2* __restrict__ cells;     // per grid cell: first entry, entries
+  const uint2* __restrict__ entries;   // lower bound of the distance from the cell (ascending), compact index | rare
   const ft_program* __restrict__ programs;
   const ft_instr* __restrict__ instrs;
   const ft_material* __restrict__ materials;
@@ -75,11 +94,7 @@ struct DevScene {
   const int32_t* __restrict__ node_op_begin;
   const int32_t* __restrict__ node_op_end;
   const int32_t* __restrict__ ur_inner_blend;
-  const float* __restrict__ ur_cell_gaps;   // per cell entry: box gap lower bound (ascending per cell)
-  const int32_t* __restrict__ ur_inner_up;  // parent link (parent << 1 | side), -1 at the root
-  const int32_t* __restrict__ ur_prim_up;   // per primitive position: parent link
   const int32_t* __restrict__ obj_node;     // per object id: the node carrying its transform, -1 none
-  const int32_t* __restrict__ ur_cell_nodes;  // per cell entry: the primitive's node index
   int32_t n_obj_node;
   int32_t n_materials, n_lights, env_program;
   int32_t bvh_root;
@@ -213,6 +228,16 @@ struct Ctx {
 
 __device__ __forceinline__ float node_lb(F3 p, const float* mn, const float* mx) { return ftd::aabb_lb(p, mn, mx); }
 
+// Object and material id of an evaluation's surface.
+__device__ __forceinline__ uint2 surface_ids(const DevScene& S, int32_t ref) {
+  if (ref == ftd::kNoRef) return make_uint2(0u, 0u);
+  const int node = ref >= 0 ? ref : __float_as_int(__ldg(S.cprims + 3 * static_cast<size_t>(~ref) + 2).z);
+  return make_uint2(S.nodes[node].object_id, S.nodes[node].material_id);
+}
+
+// A primitive of a kind without a compact record, out of line.
+__device__ __noinline__ float rare_distance(const DevNode& n, F3 p) { return ftd::prim_distance(n, p); }
+
 // eval_custom_sdf_distance (R:6139-6180) of a Custom node (a user `sdf`
 // definition): the point in its frame, through domain(p) when present, into
 // distance(p), then distance_post(d, p) when present.  The device node keeps
@@ -244,7 +269,7 @@ __device__ __noinline__ Info eval_generic(const DevScene& S, int first, int coun
     switch (op) {
       case ftgpu::kGPrim:
         cx.prim();
-        vs[vsp++] = Info{ftd::prim_distance(n, ps[psp]), n.object_id, n.material_id};
+        vs[vsp++] = Info{ftd::prim_distance(n, ps[psp]), static_cast<int32_t>(w & ftgpu::kGNodeMask)};
         break;
       case ftgpu::kGDomainPush: {
         F3 q = ftd::to_local(ps[psp], n);
@@ -282,7 +307,7 @@ __device__ __noinline__ Info eval_generic(const DevScene& S, int first, int coun
         break;
       }
       case ftgpu::kGSmooth: vs[vsp - 1].d -= n.f[0] * 0.1f; break;
-      case ftgpu::kGCustom: vs[vsp++] = Info{custom_distance(S, n, ps[psp], cx), n.object_id, n.material_id}; break;
+      case ftgpu::kGCustom: vs[vsp++] = Info{custom_distance(S, n, ps[psp], cx), static_cast<int32_t>(w & ftgpu::kGNodeMask)}; break;
     }
   }
   return vs[0];
@@ -300,144 +325,183 @@ __device__ __noinline__ Info eval_generic(const DevScene& S, int first, int coun
 // N is gathered through a BVH over the tree's primitives with pruning bound
 // max(r, min(best so far, cutoff)); primitive AABBs bound their distances from
 // below, so no primitive that can change the result is skipped.
-template <bool kStats>
-__device__ __noinline__ Info ur_fold(const DevScene& S, const DevUrTree& t, const int* near_pos,
-                                     const Info* near_info, int nn, Ctx<kStats>& cx);
+//
+// The restricted fold runs along root paths: a primitive's path gives the
+// side taken at each depth, so the lowest common ancestor of two primitives is
+// where their paths first differ, and no node is loaded on the way.
 
-// Parent value of a node whose only child holding a near primitive is on
-// `side`: the other child is +inf (exact for any far subtree, see above).
-__device__ __forceinline__ Info ur_lift(Info v, int side, float r) {
-  const Info inf{kInf, 0u, 0u};
-  return side == 0 ? ftd::combine(FT_NODE_UNION_ROUND, r, 0.0f, v, inf)
-                   : ftd::combine(FT_NODE_UNION_ROUND, r, 0.0f, inf, v);
+// Primitive `idx` of the compact array at p.
+template <bool kStats>
+__device__ __forceinline__ float compact_at(const DevScene& S, uint32_t entry, F3 p, Ctx<kStats>& cx) {
+  cx.prim();
+  const float4* w = S.cprims + 3 * static_cast<size_t>(entry & ~ftd::kRareFlag);
+  const float4 c = __ldg(w + 2);
+  if (entry & ftd::kRareFlag) return rare_distance(S.nodes[__float_as_int(c.z)], p);
+  return ftd::compact_distance(__ldg(w), __ldg(w + 1), c.x, c.y, p);
 }
 
-// The restricted fold for one or two near primitives, in registers: lift each
-// along its parent links to their lowest common ancestor, combine there, and
-// lift the result to the root.  The same operations in the same order as the
-// frame walk of ur_fold.
+// Value one level up of a subtree whose sibling holds no near primitive: the
+// other child is +inf (exact for any far subtree, see above), on either side.
+__device__ __forceinline__ float ur_lift(float v, float r) { return ftd::op_union_round(v, kInf, r); }
+
+// `levels` lifts.  Once a lift returns its input unchanged, every further one
+// does too, so the walk ends.
 template <bool kStats>
-__device__ __forceinline__ Info ur_fold_small(const DevScene& S, const DevUrTree& t, int p0, Info v0, int p1, Info v1,
-                                              int nn, Ctx<kStats>& cx) {
-  const float r = t.r;
-  int link = S.ur_prim_up[t.prim_first + p0];
-  if (nn == 2) {
-    if (p1 < p0) {  // in-order: the smaller position is in the left subtree of the common ancestor
-      int tp = p0; p0 = p1; p1 = tp;
-      Info tv = v0; v0 = v1; v1 = tv;
-      link = S.ur_prim_up[t.prim_first + p0];
-    }
-    // lift p0 until its parent's range holds p1
-    for (int guard = 0; guard <= ftgpu::kMaxUrDepth; ++guard) {
-      const DevUrInner& in = S.ur_inner[link >> 1];
-      if (in.lo <= p1 && p1 < in.hi) break;
-      v0 = ur_lift(v0, link & 1, r);
-      cx.blend();
-      link = S.ur_inner_up[link >> 1];
-    }
-    const int lca = link >> 1;
-    int l1 = S.ur_prim_up[t.prim_first + p1];
-    for (int guard = 0; guard <= ftgpu::kMaxUrDepth && (l1 >> 1) != lca; ++guard) {
-      v1 = ur_lift(v1, l1 & 1, r);
-      cx.blend();
-      l1 = S.ur_inner_up[l1 >> 1];
-    }
-    v0 = ftd::combine(FT_NODE_UNION_ROUND, r, 0.0f, v0, v1);
+__device__ __forceinline__ float ur_lifts(float v, int levels, float r, Ctx<kStats>& cx) {
+  for (int k = 0; k < levels; ++k) {
+    const float lifted = ur_lift(v, r);
     cx.blend();
-    link = S.ur_inner_up[lca];
+    if (lifted == v) break;
+    v = lifted;
   }
-  // Above the last near subtree every ancestor lifts the value the same way
-  // (either side, the other child is inert): once a lift returns its input
-  // unchanged, every further lift does too, so the walk to the root ends.
-  for (int guard = 0; guard <= ftgpu::kMaxUrDepth && link >= 0; ++guard) {
-    const Info lifted = ur_lift(v0, link & 1, r);
-    cx.blend();
-    if (lifted.d == v0.d) break;
-    v0 = lifted;
-    link = S.ur_inner_up[link >> 1];
-  }
-  return v0;
+  return v;
 }
 
-// The candidate walk and fold of eval_urtree: over the cell list [k, end)
-// (kFar false) or over the tree's BVH (kFar true).
-template <bool kStats, bool kFar>
-__device__ __forceinline__ Info eval_urtree_walk(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
-                                                 uint32_t k, uint32_t end, Ctx<kStats>& cx) {
-  const float r = t.r;
-  // near set: the first two entries in registers, the rest (rare) in arrays
-  int np0 = 0, np1 = 0;
-  Info ni0{kInf, 0u, 0u}, ni1{kInf, 0u, 0u};
-  int near_pos[ftgpu::kUrNear];
-  Info near_info[ftgpu::kUrNear];
-  int nn = 0;
-  bool overflow = false;
-  Info best{kInf, 0u, 0u};
-  // Test one primitive against the running bound; evaluate it if it can
-  // matter and record it in the near set when closer than r.
-  auto consider = [&](int pos, int node) {
-    const DevNode& pn = S.nodes[node];
-    cx.box();
-    float lim = ftd::rmax(r, fminf(best.d, cutoff));
-    if (node_lb(p, pn.bmin, pn.bmax) >= lim) return;
-    cx.prim();
-    float d = ftd::prim_distance(pn, p);
-    if (d < best.d) best = Info{d, pn.object_id, pn.material_id};
+// Depth at which two root paths part.
+__device__ __forceinline__ int ur_lca(uint4 a, uint4 b) {
+  const uint32_t lo = a.x ^ b.x, hi = a.y ^ b.y;
+  return lo ? __ffs(static_cast<int>(lo)) - 1 : 31 + __ffs(static_cast<int>(hi));
+}
+
+// op_union_round of two subtrees, the ids of the smaller child (combine).
+__device__ __forceinline__ Info ur_join(Info l, Info r, float radius) {
+  return Info{ftd::op_union_round(l.d, r.d, radius), l.d <= r.d ? l.ref : r.ref};
+}
+
+// The fold for three or more near primitives, out of line: sorted by in-order
+// position they are joined deepest common ancestor first, holding the subtrees
+// whose right part is still open on a stack.
+template <bool kStats>
+__device__ __noinline__ Info ur_fold_many(const DevScene& S, float r, int* idx, float* dist, int nn,
+                                          Ctx<kStats>& cx) {
+  for (int i = 1; i < nn; ++i) {
+    const int ki = idx[i];
+    const float kd = dist[i];
+    int j = i - 1;
+    for (; j >= 0 && idx[j] > ki; --j) {
+      idx[j + 1] = idx[j];
+      dist[j + 1] = dist[j];
+    }
+    idx[j + 1] = ki;
+    dist[j + 1] = kd;
+  }
+  Info open[ftgpu::kUrNear];
+  int at[ftgpu::kUrNear];  // depth of the ancestor that joins open[k] with what follows
+  int sp = 0;
+  uint4 path = __ldg(S.ur_paths + idx[0]);
+  Info cur{0.0f, ftd::kNoRef};
+  for (int i = 0; i < nn; ++i) {
+    cur = Info{dist[i], ~idx[i]};
+    int dep = static_cast<int>(path.z), l = -1;
+    if (i + 1 < nn) {
+      const uint4 nxt = __ldg(S.ur_paths + idx[i + 1]);
+      l = ur_lca(path, nxt);
+      path = nxt;
+    }
+    while (sp > 0 && at[sp - 1] > l) {
+      --sp;
+      cur.d = ur_lifts(cur.d, dep - at[sp] - 1, r, cx);
+      cur = ur_join(open[sp], cur, r);
+      cx.blend();
+      dep = at[sp];
+    }
+    cur.d = ur_lifts(cur.d, dep - l - 1, r, cx);
+    if (l >= 0) {
+      open[sp] = cur;
+      at[sp++] = l;
+    }
+  }
+  return cur;
+}
+
+// The fold for one or two near primitives, in registers.
+template <bool kStats>
+__device__ __forceinline__ Info ur_fold_small(const DevScene& S, float r, int i0, float d0, int i1, float d1, int nn,
+                                              Ctx<kStats>& cx) {
+  const uint4 a = __ldg(S.ur_paths + i0);
+  if (nn == 1) return Info{ur_lifts(d0, static_cast<int>(a.z), r, cx), ~i0};
+  const uint4 b = __ldg(S.ur_paths + i1);
+  const int l = ur_lca(a, b);
+  const Info v0{ur_lifts(d0, static_cast<int>(a.z) - l - 1, r, cx), ~i0};
+  const Info v1{ur_lifts(d1, static_cast<int>(b.z) - l - 1, r, cx), ~i1};
+  Info v = i0 < i1 ? ur_join(v0, v1, r) : ur_join(v1, v0, r);  // the smaller position is in the left subtree
+  cx.blend();
+  v.d = ur_lifts(v.d, l, r, cx);
+  return v;
+}
+
+// The near set of a union_round tree at a point: the nearest primitive, and
+// those closer than r: the first two in registers, further ones, rare, in the
+// caller's arrays (idx, dist; they are handed to the out-of-line fold, which
+// would otherwise put the whole set into local memory).
+struct UrNear {
+  Info best{kInf, ftd::kNoRef};
+  int i0 = 0, i1 = 0, nn = 0;
+  float d0 = 0.0f, d1 = 0.0f;
+  __device__ __forceinline__ void add(int i, float d, float r, int* idx, float* dist) {
+    if (d < best.d) best = Info{d, ~i};
     if (d < r) {
-      Info v{d, pn.object_id, pn.material_id};
       if (nn == 0) {
-        np0 = pos; ni0 = v;
+        i0 = i;
+        d0 = d;
       } else if (nn == 1) {
-        np1 = pos; ni1 = v;
+        i1 = i;
+        d1 = d;
       } else if (nn < ftgpu::kUrNear) {
-        near_pos[nn] = pos; near_info[nn] = v;
-      } else {
-        overflow = true;
-        return;
+        idx[nn] = i;
+        dist[nn] = d;
       }
       ++nn;
     }
-  };
+  }
+  // limit below which a primitive still matters
+  __device__ __forceinline__ float limit(float r, float cutoff) const { return ftd::rmax(r, fminf(best.d, cutoff)); }
+};
+
+// Tree value from its near set.
+template <bool kStats>
+__device__ __forceinline__ Info ur_value(const DevScene& S, const DevUrTree& t, const UrNear& n, int* idx,
+                                         float* dist, F3 p, Ctx<kStats>& cx) {
+  if (n.nn == 0) return n.best;
+  if (n.nn <= 2) return ur_fold_small(S, t.r, n.i0, n.d0, n.i1, n.d1, n.nn, cx);
+  if (n.nn > ftgpu::kUrNear) return eval_generic(S, t.fallback_first, t.fallback_count, p, cx);
+  idx[0] = n.i0;
+  dist[0] = n.d0;
+  idx[1] = n.i1;
+  dist[1] = n.d1;
+  return ur_fold_many(S, t.r, idx, dist, n.nn, cx);
+}
+
+// Points outside both candidate grids walk the tree's BVH, out of line: it is
+// rare beside the grids' cell walks, whose code stays in the march loops.
+template <bool kStats>
+__device__ __noinline__ Info eval_urtree_far(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
+                                             Ctx<kStats>& cx) {
+  UrNear n;
+  int near_idx[ftgpu::kUrNear];
+  float near_dist[ftgpu::kUrNear];
   int stack[48];
   int sp = 0;
-  // Candidates come from one cell list of the grid or, outside the grids,
-  // from the tree's BVH.  Both feed a single `consider` site, so the
-  // primitive evaluator is inlined once.  The cell list is sorted by a lower
-  // bound of the box bound of its points, so the first entry at or above the
-  // running limit ends it: every later primitive would be skipped by that
-  // test.
-  constexpr bool in_grid = !kFar;
-  const int32_t* list = kFar ? S.ur_bvh_prims : S.ur_cell_prims;
-  if (kFar) stack[sp++] = t.bvh_root;
-  for (int walk = 0; walk < ftgpu::kMaxWalk; ++walk) {  // each list entry and BVH node is visited once
-    if (k < end) {
-      if (in_grid) {
-        cx.cand();
-        if (S.ur_cell_gaps[k] >= ftd::rmax(r, fminf(best.d, cutoff))) break;
-      }
-      // a cell entry carries its node index; a BVH leaf's goes through ur_prims
-      const int pos = list[k];
-      consider(pos, in_grid ? S.ur_cell_nodes[k] : S.ur_prims[t.prim_first + pos]);
-      ++k;
-      continue;
-    }
-    if (in_grid || sp == 0) break;
+  stack[sp++] = t.bvh_root;
+  for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
     const DevUrBvh& bn = S.ur_bvh[stack[--sp]];
     cx.box();
-    float bound = ftd::rmax(r, fminf(best.d, cutoff));
-    if (node_lb(p, bn.bmin, bn.bmax) >= bound) continue;
+    if (node_lb(p, bn.bmin, bn.bmax) >= n.limit(t.r, cutoff)) continue;
     if (bn.prim_count > 0) {
-      k = static_cast<uint32_t>(bn.prim_begin);
-      end = k + static_cast<uint32_t>(bn.prim_count);
+      for (int k = 0; k < bn.prim_count; ++k) {
+        const int idx = t.prim_first + S.ur_bvh_prims[bn.prim_begin + k];
+        const DevNode& pn = S.nodes[S.ur_prims[idx]];
+        cx.box();
+        if (node_lb(p, pn.bmin, pn.bmax) >= n.limit(t.r, cutoff)) continue;
+        const uint32_t rare = __float_as_uint(__ldg(S.cprims + 3 * static_cast<size_t>(idx) + 2).w) & ftd::kRareFlag;
+        n.add(idx, compact_at(S, static_cast<uint32_t>(idx) | rare, p, cx), t.r, near_idx, near_dist);
+      }
       continue;
     }
     const DevUrBvh& L = S.ur_bvh[bn.left];
     const DevUrBvh& R = S.ur_bvh[bn.right];
     float ll = node_lb(p, L.bmin, L.bmax), rl = node_lb(p, R.bmin, R.bmax);
-    if (sp + 2 > 48) {
-      overflow = true;
-      break;
-    }
+    if (sp + 2 > 48) return eval_generic(S, t.fallback_first, t.fallback_count, p, cx);
     if (ll <= rl) {
       stack[sp++] = bn.right;
       stack[sp++] = bn.left;
@@ -446,111 +510,60 @@ __device__ __forceinline__ Info eval_urtree_walk(const DevScene& S, const DevUrT
       stack[sp++] = bn.right;
     }
   }
-  if (overflow) return eval_generic(S, t.fallback_first, t.fallback_count, p, cx);
-  if (nn == 0) return best;
-  if (nn <= 2) return ur_fold_small(S, t, np0, ni0, np1, ni1, nn, cx);
-  near_pos[0] = np0; near_info[0] = ni0;
-  near_pos[1] = np1; near_info[1] = ni1;
-  return ur_fold(S, t, near_pos, near_info, nn, cx);
+  return ur_value(S, t, n, near_idx, near_dist, p, cx);
 }
 
-// Points outside both candidate grids walk the tree's BVH, out of line: it is
-// rare beside the grids' cell walks, whose code stays in the march loops.
+// Cell of p in a grid; false outside it.
+__device__ __forceinline__ bool grid_cell(const DevGrid& g, F3 p, int* cell) {
+  const float gx = (p.x - g.gmin[0]) * g.inv_cell, gy = (p.y - g.gmin[1]) * g.inv_cell,
+              gz = (p.z - g.gmin[2]) * g.inv_cell;
+  if (!(gx >= 0.0f && gy >= 0.0f && gz >= 0.0f && gx < (float)g.dims[0] && gy < (float)g.dims[1] &&
+        gz < (float)g.dims[2]))
+    return false;
+  const int ix = min((int)gx, g.dims[0] - 1), iy = min((int)gy, g.dims[1] - 1), iz = min((int)gz, g.dims[2] - 1);
+  *cell = g.first + ix + g.dims[0] * (iy + g.dims[1] * iz);
+  return true;
+}
+
+// A walk is bound by the latency of its three dependent loads (cell, entry,
+// primitive) and the branches between them, so each is one vector load of a
+// compact record and the distance has no branch.  With the scene's header in
+// the constant bank, the 512-primitive field's depth frame (1920x1080, 2x2)
+// takes 11.9 ms, against 29.8 ms with scalar loads from 128-byte nodes, a box
+// test per candidate and parent-link folds.
+//
+// The tree's value at p, exact where it is below `cutoff`: the candidates of
+// p's cell in the fine grid, or outside it in the coarser outer grid around it
+// (its cells list the primitives that can be the nearest there), else the
+// tree's BVH.  A cell's list is sorted by a lower bound of its points'
+// distances, so the first entry at or above the running limit ends it.
 template <bool kStats>
-__device__ __noinline__ Info eval_urtree_far(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
-                                             Ctx<kStats>& cx) {
-  return eval_urtree_walk<kStats, true>(S, t, p, cutoff, 0u, 0u, cx);
-}
-
-// kFarCall: the BVH walk for points outside both grids is the out-of-line
-// eval_urtree_far (the march loops), or inlined here (the shadow loop, whose
-// 64-register budget measured 16 % slower with the call: 71.5 against 60.3 ms
-// per 1920x1080 Whitted frame of the 512-primitive union_round field, while
-// the march kernel gained 3 %).
-template <bool kStats, bool kFarCall = true>
 __device__ __forceinline__ Info eval_urtree(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
                                             Ctx<kStats>& cx) {
-  // The fine grid, outside it the coarser outer grid around it (its cells
-  // list the primitives that can be the nearest there), else the BVH.
-  float gx = (p.x - t.gmin[0]) * t.inv_cell, gy = (p.y - t.gmin[1]) * t.inv_cell, gz = (p.z - t.gmin[2]) * t.inv_cell;
-  int gd0 = t.dims[0], gd1 = t.dims[1], gd2 = t.dims[2], gfirst = t.cell_first;
-  bool in_grid = gd0 > 0 && gx >= 0.0f && gy >= 0.0f && gz >= 0.0f && gx < (float)gd0 && gy < (float)gd1 &&
-                 gz < (float)gd2;
-  if (!in_grid && t.odims[0] > 0) {
-    gx = (p.x - t.ogmin[0]) * t.oinv_cell;
-    gy = (p.y - t.ogmin[1]) * t.oinv_cell;
-    gz = (p.z - t.ogmin[2]) * t.oinv_cell;
-    gd0 = t.odims[0];
-    gd1 = t.odims[1];
-    gd2 = t.odims[2];
-    gfirst = t.ocell_first;
-    in_grid = gx >= 0.0f && gy >= 0.0f && gz >= 0.0f && gx < (float)gd0 && gy < (float)gd1 && gz < (float)gd2;
-  }
-  if (!in_grid) return kFarCall ? eval_urtree_far(S, t, p, cutoff, cx) : eval_urtree_walk<kStats, true>(S, t, p, cutoff, 0u, 0u, cx);
-  const int ix = min((int)gx, gd0 - 1), iy = min((int)gy, gd1 - 1), iz = min((int)gz, gd2 - 1);
-  const int cell = gfirst + ix + gd0 * (iy + gd1 * iz);
-  return eval_urtree_walk<kStats, false>(S, t, p, cutoff, S.ur_cell_offsets[cell], S.ur_cell_offsets[cell + 1], cx);
-}
-
-// Restricted union_round fold over the subtrees holding near primitives
-// (out of line: only points within r of a primitive take it).
-template <bool kStats>
-__device__ __noinline__ Info ur_fold(const DevScene& S, const DevUrTree& t, const int* near_pos,
-                                     const Info* near_info, int nn, Ctx<kStats>& cx) {
+  int cell = 0;
+  if (!grid_cell(t.fine, p, &cell) && !grid_cell(t.outer, p, &cell)) return eval_urtree_far(S, t, p, cutoff, cx);
+  const uint2 range = __ldg(S.cells + cell);
   const float r = t.r;
-  // Frames hold partially combined inner nodes.
-  struct Frame {
-    int inner, stage;
-    Info slot[2];
-  };
-  Frame fr[ftgpu::kMaxUrDepth + 1];
-  int fp = 0;
-  fr[0].inner = t.inner_root;
-  fr[0].stage = 0;
-  for (int walk = 0; walk < ftgpu::kMaxWalk; ++walk) {  // each inner node is opened once
-    Frame& F = fr[fp];
-    if (F.stage < 2) {
-      const DevUrInner& in = S.ur_inner[F.inner];
-      int c = in.child[F.stage];
-      if (c < 0) {
-        int pos = -c - 1;
-        Info v{kInf, 0u, 0u};
-        for (int k = 0; k < nn; ++k)
-          if (near_pos[k] == pos) v = near_info[k];
-        F.slot[F.stage++] = v;
-        continue;
-      }
-      const DevUrInner& ci = S.ur_inner[c];
-      bool has = false;
-      for (int k = 0; k < nn; ++k) has |= (near_pos[k] >= ci.lo && near_pos[k] < ci.hi);
-      if (!has) {
-        F.slot[F.stage++] = Info{kInf, 0u, 0u};
-        continue;
-      }
-      if (fp + 1 > ftgpu::kMaxUrDepth) break;  // deeper than the builder admits
-      ++F.stage;
-      ++fp;
-      fr[fp].inner = c;
-      fr[fp].stage = 0;
-      continue;
-    }
-    Info res = ftd::combine(FT_NODE_UNION_ROUND, r, 0.0f, F.slot[0], F.slot[1]);
-    cx.blend();
-    if (fp == 0) return res;
-    --fp;
-    fr[fp].slot[fr[fp].stage - 1] = res;
+  UrNear n;
+  int near_idx[ftgpu::kUrNear];
+  float near_dist[ftgpu::kUrNear];
+  for (uint32_t k = range.x, end = range.x + range.y; k < end; ++k) {
+    const uint2 e = __ldg(S.entries + k);
+    cx.cand();
+    if (__uint_as_float(e.x) >= n.limit(r, cutoff)) break;
+    n.add(static_cast<int>(e.y & ~ftd::kRareFlag), compact_at(S, e.y, p, cx), r, near_idx, near_dist);
   }
-  return Info{kInf, 0u, 0u};  // only a corrupted tree gets here
+  return ur_value(S, t, n, near_idx, near_dist, p, cx);
 }
 
-template <bool kStats, bool kFarCall = true>
+template <bool kStats>
 __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, F3 p, float cutoff, Ctx<kStats>& cx) {
   if (lf.kind == ftgpu::kLeafPrim) {
     const DevNode& n = S.nodes[lf.node];
     cx.prim();
-    return Info{ftd::prim_distance(n, p), n.object_id, n.material_id};
+    return Info{ftd::prim_distance(n, p), lf.node};
   }
-  if (lf.kind == ftgpu::kLeafUrTree) return eval_urtree<kStats, kFarCall>(S, S.urtrees[lf.first], p, cutoff, cx);
+  if (lf.kind == ftgpu::kLeafUrTree) return eval_urtree(S, S.urtrees[lf.first], p, cutoff, cx);
   if (S.nodes[lf.node].kind == FT_NODE_CUSTOM) {
     // accel_leaf_distance_info (R:635-657): a Custom leaf farther from its box
     // than a tenth of the box diagonal (clamped to [0.05, 0.5]) is that box
@@ -560,7 +573,7 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, 
     float lb = node_lb(p, lf.bmin, lf.bmax);
     float ex = lf.bmax[0] - lf.bmin[0], ey = lf.bmax[1] - lf.bmin[1], ez = lf.bmax[2] - lf.bmin[2];
     float far = ftd::rclamp(sqrtf(ex * ex + ey * ey + ez * ez) * 0.1f, 0.05f, 0.5f);
-    if (lb > far) return Info{lb, n.object_id, n.material_id};
+    if (lb > far) return Info{lb, lf.node};
   }
   return eval_generic(S, lf.first, lf.count, p, cx);
 }
@@ -572,7 +585,7 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, 
 template <bool kStats>
 __device__ __noinline__ Info scene_distance_bvh(const DevScene& S, F3 p, Ctx<kStats>& cx) {
   float best = kInf;
-  Info cur{kInf, 0u, 0u};
+  Info cur{kInf, ftd::kNoRef};
   int stack[64];
   float stack_lb[64];
   int sp = 0;
@@ -615,13 +628,13 @@ __device__ __noinline__ Info scene_distance_bvh(const DevScene& S, F3 p, Ctx<kSt
 // evaluation site for both leaves: the leaf evaluator (with the whole
 // union_round path) is inlined once, which keeps the march loops' code within
 // the instruction cache.
-template <bool kStats, bool kFarCall = true>
+template <bool kStats>
 __device__ __forceinline__ Info scene_distance_leaves(const DevScene& S, F3 p, int leaf, int second, float second_lb,
                                                       Ctx<kStats>& cx) {
-  Info cur{kInf, 0u, 0u};
+  Info cur{kInf, ftd::kNoRef};
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
-    const Info in = eval_leaf<kStats, kFarCall>(S, S.leaves[leaf], p, k == 0 ? kInf : cur.d, cx);
+    const Info in = eval_leaf(S, S.leaves[leaf], p, k == 0 ? kInf : cur.d, cx);
     if (k == 0 || in.d < cur.d) cur = in;
     if (second < 0 || !(second_lb <= cur.d)) break;
     leaf = second;
@@ -632,8 +645,7 @@ __device__ __forceinline__ Info scene_distance_leaves(const DevScene& S, F3 p, i
 // Same traversal, with the one- and two-leaf BVHs (a single object, or a
 // ground plus one composite object) walked without a stack.
 template <bool kStats>
-__device__ __forceinline__ Info scene_distance_inl(const DevScene& S, F3 p, Ctx<kStats>& cx) {
-  cx.eval();
+__device__ __noinline__ Info scene_distance_general(const DevScene& S, F3 p, Ctx<kStats>& cx) {
   const DevBvhNode& root = S.bvh[S.bvh_root];
   int leaf = root.leaf, second = -1;
   float second_lb = kInf;
@@ -649,6 +661,37 @@ __device__ __forceinline__ Info scene_distance_inl(const DevScene& S, F3 p, Ctx<
     second_lb = lfirst ? rl : ll;
   }
   return scene_distance_leaves(S, p, leaf, second, second_lb, cx);
+}
+
+// kFastTree with a primitive leaf: the two-leaf walk above (nearer box first,
+// the other leaf when its box bound is not above the distance found) with the
+// primitive evaluated first in either order, so that its distance bounds the
+// tree's walk.  t2 and p2 are the squared box bounds of the tree and the
+// primitive.  Where the tree comes first it is exact below the cutoff, and at
+// or above it the primitive's distance wins as it would there; a negative
+// primitive distance (a point inside it) does not cut the walk.
+template <bool kStats>
+__device__ __forceinline__ Info tree_and_prim(const DevScene& S, F3 p, float t2, float p2, Ctx<kStats>& cx) {
+  const DevFast& F = S.fast;
+  const bool tree_first = F.tree_lhs ? t2 <= p2 : t2 < p2;
+  const Info prim{compact_at(S, F.prim, p, cx), ~static_cast<int32_t>(F.prim & ~ftd::kRareFlag)};
+  if (!tree_first && !(sqrtf(t2) <= prim.d)) return prim;
+  const Info tree = eval_urtree(S, F.tree, p, tree_first && prim.d < 0.0f ? kInf : prim.d, cx);
+  if (!tree_first) return tree.d < prim.d ? tree : prim;
+  return prim.d < tree.d && sqrtf(p2) <= tree.d ? prim : tree;
+}
+
+// The scene distance at p (Accelerator::distance_info): the short form of the
+// scene's kind inline in the march loops, every other scene out of line, so
+// that the loops' code stays small.
+template <bool kStats>
+__device__ __forceinline__ Info scene_distance_inl(const DevScene& S, F3 p, Ctx<kStats>& cx) {
+  cx.eval();
+  const DevFast& F = S.fast;
+  if (F.kind != kFastTree) return scene_distance_general(S, p, cx);
+  if (F.prim == kNoPrim) return eval_urtree(S, F.tree, p, kInf, cx);
+  cx.box(2);
+  return tree_and_prim(S, p, ftd::aabb_lb2(p, F.tmin, F.tmax), ftd::aabb_lb2(p, F.pmin, F.pmax), cx);
 }
 
 template <bool kStats>
@@ -668,7 +711,7 @@ template <bool kStats>
 __device__ __noinline__ Info scene_distance_leaf(const DevScene& S, F3 p, int* leaf, Ctx<kStats>& cx) {
   cx.eval();
   float best = kInf;
-  Info cur{kInf, 0u, 0u};
+  Info cur{kInf, ftd::kNoRef};
   *leaf = 0;
   int stack[64];
   float stack_lb[64];
@@ -771,7 +814,7 @@ __device__ HitOut march(const DevScene& S, const RayParams& P, F3 o, F3 d, bool 
       }
       Info fin = scene_distance(S, pos, cx);
       h.t = hi;
-      h.mat = fin.mat;
+      h.mat = surface_ids(S, fin.ref).y;
       h.hit = true;
       return h;
     }
@@ -818,7 +861,8 @@ __device__ __forceinline__ uint32_t batch_item(const BatchView& V, uint64_t g) {
 }
 
 template <bool kStats>
-__global__ void __launch_bounds__(128) march_depth_kernel(DevScene S, RayParams P, float* __restrict__ t_out,
+__global__ void __launch_bounds__(128) march_depth_kernel(const __grid_constant__ DevScene S,
+                                                          const __grid_constant__ RayParams P, float* __restrict__ t_out,
                                                           uint8_t* __restrict__ mask_out,
                                                           uint32_t* __restrict__ mat_out,
                                                           float* __restrict__ normal_out,
@@ -858,6 +902,7 @@ __global__ void __launch_bounds__(128) march_depth_kernel(DevScene S, RayParams 
 // Primary ray of work item i (pixel_sample_offsets R:4838-4854, NDC map of
 // render_depth_tile R:3951-3955, generate_ray render_api.rs:132-144 and the
 // second normalisation of the tile loop).
+template <bool kYFirst = false>
 __device__ __forceinline__ bool item_ray(const RayParams& P, uint64_t i, F3* dir, size_t* out_idx) {
   uint32_t px, py, s;
   item_coords(P, i, &px, &py, &s);
@@ -867,8 +912,8 @@ __device__ __forceinline__ bool item_ray(const RayParams& P, uint64_t i, F3* dir
   ndc_x *= P.aspect;
   F3 fwd = f3(P.fwd[0], P.fwd[1], P.fwd[2]), rt = f3(P.right[0], P.right[1], P.right[2]);
   F3 up = f3(P.up[0], P.up[1], P.up[2]);
-  F3 d = ftd::normalize3(fwd + rt * (ndc_x * P.tan_fov) + up * (ndc_y * P.tan_fov));
-  *dir = ftd::normalize3(d);
+  F3 d = ftd::normalize3_fma<false>(fwd + rt * (ndc_x * P.tan_fov) + up * (ndc_y * P.tan_fov));
+  *dir = ftd::normalize3_fma<kYFirst>(d);
   *out_idx = (static_cast<size_t>(py) * P.width + px) * P.aa + s;
   return true;
 }
@@ -911,13 +956,20 @@ constexpr unsigned long long kMarchWallNs = 20ull * 1000000000ull;  // per warp
 // (80 registers), 161 with four, 148 with the compiler's own choice (64
 // registers and more spills) and 132 with one block (123 registers).
 template <bool kStats, bool kBricks, bool kBatch>
-__global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, RayParams P0, DevBricks B0, BatchView V,
+__global__ void __launch_bounds__(128, 5) march_depth_persistent(
+    const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ DevBricks B0,
+    const __grid_constant__ BatchView V,
                                                               float* __restrict__ t_out,
                                                               uint8_t* __restrict__ mask_out,
                                                               uint32_t* __restrict__ mat_out,
                                                               float* __restrict__ normal_out,
                                                               unsigned long long* __restrict__ stats,
                                                               unsigned long long* __restrict__ next_item) {
+#ifdef FT_JIT
+  constexpr bool kRayYFirst = true;
+#else
+  constexpr bool kRayYFirst = kBricks && !kBatch;
+#endif
   const unsigned lane = threadIdx.x & 31u;
   const bool want_normal = normal_out != nullptr;
   const uint64_t n_work = kBatch ? V.n_rays : P0.n_items;
@@ -1003,7 +1055,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, Ra
           if (kBatch) {
             item_of_lane = batch_item(V, item);
             const RayParams& Pi = V.params[item_of_lane];
-            got = item_ray(Pi, item - V.ray_first[item_of_lane], &d, &idx);
+            got = item_ray<kRayYFirst>(Pi, item - V.ray_first[item_of_lane], &d, &idx);
             idx += V.out_first[item_of_lane];
             o = f3(Pi.origin[0], Pi.origin[1], Pi.origin[2]);
             eps = Pi.eps;
@@ -1011,7 +1063,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, Ra
             min_step = fmaxf(eps * 0.5f, 1.0e-5f);
             ne = fmaxf(eps * 4.0f, 1.0e-5f);
           } else {
-            got = item_ray(P0, item, &d, &idx);
+            got = item_ray<kRayYFirst>(P0, item, &d, &idx);
           }
         }
         const DevScene& S = kBatch ? V.scenes[item_of_lane] : S0;
@@ -1113,7 +1165,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, Ra
       } else {
         // the nearest leaf is the ground and the ray descends: the cached
         // bound decides whether the rest of the approach is a plane descent
-        if (kBricks && !B.free_far && B.plane_leaf >= 0 && info.obj == B.plane_obj && d.y < 0.0f &&
+        if (kBricks && !B.free_far && B.plane_leaf >= 0 && d.y < 0.0f && surface_ids(S, info.ref).x == B.plane_obj &&
             plane_jump(B, q, d, info.d, cached_lb(B, q, cx), eps, scale, min_step)) {
           // The rest of the plain march descends on the plane: after n more
           // steps it first samples inside the eps shell (heights shrink by
@@ -1149,7 +1201,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, Ra
       bool accept = true;
       if (fabsf(info.d) < eps) {
         hi = mid;
-        hit_mat = info.mat;
+        hit_mat = surface_ids(S, info.ref).y;
         mat_known = true;
       } else if (info.d > 0.0f && ++k < 3) {
         lo = mid;
@@ -1184,7 +1236,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(DevScene S0, Ra
         else phase = kFinal;
       }
     } else {
-      write_hit(info.mat);
+      write_hit(surface_ids(S, info.ref).y);
     }
   }
   if (kStats) flush_stats(cx.c, stats);
@@ -1485,6 +1537,7 @@ __global__ void batch_pixels_kernel(const BatchPixItem* __restrict__ items, uint
 }
 
 #include "ft_diff.cuh"
+#include "ft_grid.cuh"
 
 // Dependent-FMA chains, 8 per thread, for the FP32 roofline denominator.
 __global__ void fma_peak_kernel(float* out, int iters, float a, float b) {

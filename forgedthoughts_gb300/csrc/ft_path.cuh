@@ -52,8 +52,9 @@ __device__ bool march_hit(const DevScene& S, const RayParams& P, F3 o, F3 d, flo
       const Info fin = scene_distance_leaf(S, pos, &h->leaf, cx);
       h->t = hi;
       h->pos = pos;
-      h->mat = fin.mat;
-      h->obj = fin.obj;
+      const uint2 ids = surface_ids(S, fin.ref);
+      h->mat = ids.y;
+      h->obj = ids.x;
       return true;
     }
     prev = traveled;
@@ -431,7 +432,7 @@ __device__ F3 trace_path(const DevScene& S, const RayParams& P, F3 origin, F3 di
 // stopping.  Outputs the average (linear), its spectrum_to_rgb8 (R:5221-5227)
 // and the samples taken.
 template <bool kStats>
-__global__ void __launch_bounds__(128) path_pixel_kernel(DevScene S, RayParams P, PathSettingsD ps,
+__global__ void __launch_bounds__(128) path_pixel_kernel(const __grid_constant__ DevScene S, const __grid_constant__ RayParams P, PathSettingsD ps,
                                                          float* __restrict__ rgb_out, uint8_t* __restrict__ rgb8_out,
                                                          uint32_t* __restrict__ count_out,
                                                          unsigned long long* __restrict__ stats) {

@@ -32,7 +32,8 @@
 
 static_assert(sizeof(DevLeaf) == sizeof(ftgpu::HostLeaf), "leaf layout");
 static_assert(sizeof(DevBvhNode) == sizeof(ftgpu::HostBvhNode), "bvh layout");
-static_assert(sizeof(DevUrTree) == sizeof(ftgpu::HostUrTree), "urtree layout");
+static_assert(3 * sizeof(float4) == sizeof(ftgpu::CompactPrim), "compact primitive layout");
+static_assert(sizeof(uint4) == sizeof(ftgpu::UrPath), "root path layout");
 static_assert(sizeof(DevUrBvh) == sizeof(ftgpu::HostUrBvh), "urbvh layout");
 static_assert(sizeof(DevUrInner) == sizeof(ftgpu::HostUrInner), "urinner layout");
 
@@ -94,6 +95,10 @@ struct ft_scene {
   ftgpu::SceneImage img;
   void* arena = nullptr;
   size_t arena_bytes = 0;
+  // Candidate grids of the scene, built on the device (build_grids)
+  uint2* grid_cells = nullptr;
+  uint2* grid_entries = nullptr;
+  size_t grid_bytes = 0;
   DevScene dev{};
   // Per-render buffers, grown on demand and reused across calls.
   float* d_t = nullptr;
@@ -180,6 +185,81 @@ void prof_collect(ft_scene* sc) {
   sc->prof_pending.clear();
 }
 
+// Candidate-list entries of all grids of a scene (8 bytes each); a grid past
+// it is dropped, and its points take the tree BVH.
+constexpr uint64_t kMaxGridEntries = uint64_t(1) << 26;
+
+// Build the cell lists of `jobs` into one cell and one entry array: count,
+// read the totals, drop the grids that would pass the entry cap (their job's
+// `dims` become 0), fill.
+ft_status build_grids(ft_scene* sc, std::vector<GridJob>* jobs) {
+  uint64_t n_cells = 0;
+  for (GridJob& j : *jobs) {
+    j.first = static_cast<int32_t>(n_cells);
+    n_cells += static_cast<uint64_t>(j.dims[0]) * j.dims[1] * j.dims[2];
+  }
+  if (n_cells == 0) return FT_OK;
+  auto blocks = [](const GridJob& j) {
+    auto n = [&](int a) { return static_cast<unsigned>((j.dims[a] + kGridBlockEdge - 1) / kGridBlockEdge); };
+    return n(0) * n(1) * n(2);
+  };
+  // per job the entry total, then the fill's allocation cursor
+  const size_t n_totals = jobs->size() + 1;
+  const size_t totals_off = align_up(n_cells * sizeof(uint2), 256);
+  FT_CUDA_TRY(cudaMalloc(&sc->grid_cells, totals_off + n_totals * sizeof(unsigned long long)), "cudaMalloc(grid)");
+  auto* totals = reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(sc->grid_cells) + totals_off);
+  FT_CUDA_TRY(cudaMemsetAsync(totals, 0, n_totals * sizeof(unsigned long long)), "cudaMemset(grid)");
+  for (size_t k = 0; k < jobs->size(); ++k)
+    grid_cells_kernel<false><<<blocks((*jobs)[k]), 64>>>(sc->dev, (*jobs)[k], sc->grid_cells, nullptr, totals + k);
+  FT_CUDA_TRY(cudaGetLastError(), "grid_cells_kernel launch");
+  std::vector<unsigned long long> count(n_totals);
+  FT_CUDA_TRY(cudaMemcpy(count.data(), totals, n_totals * sizeof(unsigned long long), cudaMemcpyDeviceToHost),
+              "grid totals");
+  uint64_t entries = 0;
+  for (size_t k = 0; k < jobs->size(); ++k) {
+    if (entries + count[k] > kMaxGridEntries) (*jobs)[k].dims[0] = 0;
+    else entries += count[k];
+  }
+  FT_CUDA_TRY(cudaMalloc(&sc->grid_entries, std::max<uint64_t>(entries, 1) * sizeof(uint2)), "cudaMalloc(grid)");
+  sc->grid_bytes = totals_off + n_totals * sizeof(unsigned long long) + entries * sizeof(uint2);
+  sc->dev.cells = sc->grid_cells;
+  sc->dev.entries = sc->grid_entries;
+  for (const GridJob& j : *jobs)
+    if (j.dims[0] > 0)
+      grid_cells_kernel<true><<<blocks(j), 64>>>(sc->dev, j, sc->grid_cells, sc->grid_entries, totals + jobs->size());
+  FT_CUDA_TRY(cudaGetLastError(), "grid_cells_kernel launch");
+  FT_CUDA_TRY(cudaStreamSynchronize(nullptr), "grid build");  // renders run on any stream
+  return FT_OK;
+}
+
+// A grid's job; `slack` is far above the rounding of a few float operations on
+// its coordinates.
+GridJob grid_job(const float gmin[3], float cell, const int32_t dims[3], int32_t prim_first, int32_t n_prims, float r) {
+  GridJob j{};
+  float scale = 0.0f;
+  for (int a = 0; a < 3; ++a) {
+    j.gmin[a] = gmin[a];
+    j.dims[a] = dims[a];
+    scale = std::max({scale, std::fabs(gmin[a]), std::fabs(gmin[a] + static_cast<float>(dims[a]) * cell)});
+  }
+  j.cell = cell;
+  j.prim_first = prim_first;
+  j.n_prims = n_prims;
+  j.r = r;
+  j.slack = 1.0e-6f + 4.0e-6f * scale;
+  return j;
+}
+
+DevGrid dev_grid(const GridJob& j) {
+  DevGrid g{};
+  if (j.dims[0] <= 0) return g;
+  std::memcpy(g.gmin, j.gmin, sizeof(g.gmin));
+  std::memcpy(g.dims, j.dims, sizeof(g.dims));
+  g.inv_cell = 1.0f / j.cell;
+  g.first = j.first;
+  return g;
+}
+
 ft_status upload_scene(ft_scene* sc) {
   const ftgpu::SceneImage& im = sc->img;
   struct Part {
@@ -187,31 +267,31 @@ ft_status upload_scene(ft_scene* sc) {
     size_t bytes;
     size_t off;
   };
-  std::vector<Part> parts = {
-      {im.nodes.data(), im.nodes.size() * sizeof(DevNode), 0},
-      {im.leaves.data(), im.leaves.size() * sizeof(DevLeaf), 0},
-      {im.bvh.data(), im.bvh.size() * sizeof(DevBvhNode), 0},
-      {im.gops.data(), im.gops.size() * sizeof(uint32_t), 0},
-      {im.urtrees.data(), im.urtrees.size() * sizeof(DevUrTree), 0},
-      {im.ur_bvh.data(), im.ur_bvh.size() * sizeof(DevUrBvh), 0},
-      {im.ur_bvh_prims.data(), im.ur_bvh_prims.size() * sizeof(int32_t), 0},
-      {im.ur_prims.data(), im.ur_prims.size() * sizeof(int32_t), 0},
-      {im.ur_inner.data(), im.ur_inner.size() * sizeof(DevUrInner), 0},
-      {im.programs.data(), im.programs.size() * sizeof(ft_program), 0},
-      {im.instrs.data(), im.instrs.size() * sizeof(ft_instr), 0},
-      {im.ur_cell_offsets.data(), im.ur_cell_offsets.size() * sizeof(uint32_t), 0},
-      {im.ur_cell_prims.data(), im.ur_cell_prims.size() * sizeof(int32_t), 0},
-      {im.materials.data(), im.materials.size() * sizeof(ft_material), 0},
-      {im.lights.data(), im.lights.size() * sizeof(ft_light), 0},
-      {im.node_op_begin.data(), im.node_op_begin.size() * sizeof(int32_t), 0},
-      {im.node_op_end.data(), im.node_op_end.size() * sizeof(int32_t), 0},
-      {im.ur_inner_blend.data(), im.ur_inner_blend.size() * sizeof(int32_t), 0},
-      {im.ur_cell_gaps.data(), im.ur_cell_gaps.size() * sizeof(float), 0},
-      {im.ur_inner_up.data(), im.ur_inner_up.size() * sizeof(int32_t), 0},
-      {im.ur_prim_up.data(), im.ur_prim_up.size() * sizeof(int32_t), 0},
-      {im.obj_node.data(), im.obj_node.size() * sizeof(int32_t), 0},
-      {im.ur_cell_nodes.data(), im.ur_cell_nodes.size() * sizeof(int32_t), 0},
+  std::vector<DevUrTree> trees;
+  for (const ftgpu::HostUrTree& t : im.urtrees) {
+    DevUrTree d{};
+    d.r = t.r;
+    d.n_prims = t.n_prims;
+    d.prim_first = t.prim_first;
+    d.bvh_root = t.bvh_root;
+    d.inner_root = t.inner_root;
+    d.depth = t.depth;
+    d.fallback_first = t.fallback_first;
+    d.fallback_count = t.fallback_count;
+    trees.push_back(d);
+  }
+  std::vector<Part> parts;
+  auto part = [&](const void* src, size_t bytes) {
+    parts.push_back(Part{src, bytes, 0});
+    return parts.size() - 1;
   };
+  auto vec = [&](const auto& v) { return part(v.data(), v.size() * sizeof(v[0])); };
+  const size_t p_nodes = vec(im.nodes), p_leaves = vec(im.leaves), p_bvh = vec(im.bvh), p_gops = vec(im.gops),
+               p_trees = vec(trees), p_ur_bvh = vec(im.ur_bvh), p_ur_bvh_prims = vec(im.ur_bvh_prims),
+               p_ur_prims = vec(im.ur_prims), p_ur_inner = vec(im.ur_inner), p_programs = vec(im.programs),
+               p_instrs = vec(im.instrs), p_cprims = vec(im.cprims), p_paths = vec(im.ur_paths),
+               p_materials = vec(im.materials), p_lights = vec(im.lights), p_op_begin = vec(im.node_op_begin),
+               p_op_end = vec(im.node_op_end), p_blend = vec(im.ur_inner_blend), p_obj = vec(im.obj_node);
   size_t total = 0;
   for (Part& p : parts) {
     p.off = total;
@@ -224,37 +304,72 @@ ft_status upload_scene(ft_scene* sc) {
   sc->arena_bytes = total;
   FT_CUDA_TRY(cudaMemcpy(sc->arena, staging.data(), total, cudaMemcpyHostToDevice), "cudaMemcpy(scene)");
   unsigned char* base = static_cast<unsigned char*>(sc->arena);
+  auto at = [&](size_t k, auto& out) {
+    out = reinterpret_cast<std::remove_reference_t<decltype(out)>>(base + parts[k].off);
+  };
   DevScene& d = sc->dev;
-  d.nodes = reinterpret_cast<const DevNode*>(base + parts[0].off);
-  d.leaves = reinterpret_cast<const DevLeaf*>(base + parts[1].off);
-  d.bvh = reinterpret_cast<const DevBvhNode*>(base + parts[2].off);
-  d.gops = reinterpret_cast<const uint32_t*>(base + parts[3].off);
-  d.urtrees = reinterpret_cast<const DevUrTree*>(base + parts[4].off);
-  d.ur_bvh = reinterpret_cast<const DevUrBvh*>(base + parts[5].off);
-  d.ur_bvh_prims = reinterpret_cast<const int32_t*>(base + parts[6].off);
-  d.ur_prims = reinterpret_cast<const int32_t*>(base + parts[7].off);
-  d.ur_inner = reinterpret_cast<const DevUrInner*>(base + parts[8].off);
-  d.programs = reinterpret_cast<const ft_program*>(base + parts[9].off);
-  d.instrs = reinterpret_cast<const ft_instr*>(base + parts[10].off);
-  d.ur_cell_offsets = reinterpret_cast<const uint32_t*>(base + parts[11].off);
-  d.ur_cell_prims = reinterpret_cast<const int32_t*>(base + parts[12].off);
-  d.materials = reinterpret_cast<const ft_material*>(base + parts[13].off);
-  d.lights = reinterpret_cast<const ft_light*>(base + parts[14].off);
-  d.node_op_begin = reinterpret_cast<const int32_t*>(base + parts[15].off);
-  d.node_op_end = reinterpret_cast<const int32_t*>(base + parts[16].off);
-  d.ur_inner_blend = reinterpret_cast<const int32_t*>(base + parts[17].off);
-  d.ur_cell_gaps = reinterpret_cast<const float*>(base + parts[18].off);
-  d.ur_inner_up = reinterpret_cast<const int32_t*>(base + parts[19].off);
-  d.ur_prim_up = reinterpret_cast<const int32_t*>(base + parts[20].off);
-  d.obj_node = reinterpret_cast<const int32_t*>(base + parts[21].off);
+  at(p_nodes, d.nodes);
+  at(p_leaves, d.leaves);
+  at(p_bvh, d.bvh);
+  at(p_gops, d.gops);
+  at(p_trees, d.urtrees);
+  at(p_ur_bvh, d.ur_bvh);
+  at(p_ur_bvh_prims, d.ur_bvh_prims);
+  at(p_ur_prims, d.ur_prims);
+  at(p_ur_inner, d.ur_inner);
+  at(p_programs, d.programs);
+  at(p_instrs, d.instrs);
+  at(p_cprims, d.cprims);
+  at(p_paths, d.ur_paths);
+  at(p_materials, d.materials);
+  at(p_lights, d.lights);
+  at(p_op_begin, d.node_op_begin);
+  at(p_op_end, d.node_op_end);
+  at(p_blend, d.ur_inner_blend);
+  at(p_obj, d.obj_node);
   d.n_obj_node = static_cast<int32_t>(im.obj_node.size());
-  d.ur_cell_nodes = reinterpret_cast<const int32_t*>(base + parts[22].off);
   d.n_materials = static_cast<int32_t>(im.materials.size());
   d.n_lights = static_cast<int32_t>(im.lights.size());
   d.env_program = im.environment_program;
   d.bvh_root = im.bvh_root;
   std::memcpy(d.smin, im.scene_min, sizeof(d.smin));
   std::memcpy(d.smax, im.scene_max, sizeof(d.smax));
+  // the union_round trees' candidate grids (fine, outer)
+  std::vector<GridJob> jobs;
+  std::vector<std::pair<size_t, bool>> owner;
+  for (size_t k = 0; k < im.urtrees.size(); ++k) {
+    const ftgpu::HostUrTree& t = im.urtrees[k];
+    if (t.dims[0] <= 0) continue;
+    jobs.push_back(grid_job(t.gmin, t.cell, t.dims, t.prim_first, t.n_prims, t.r));
+    owner.emplace_back(k, false);
+    if (t.odims[0] <= 0) continue;
+    jobs.push_back(grid_job(t.ogmin, t.ocell, t.odims, t.prim_first, t.n_prims, t.r));
+    owner.emplace_back(k, true);
+  }
+  if (ft_status s = build_grids(sc, &jobs)) return s;
+  for (size_t k = 0; k < jobs.size(); ++k)
+    (owner[k].second ? trees[owner[k].first].outer : trees[owner[k].first].fine) = dev_grid(jobs[k]);
+  if (!trees.empty())
+    FT_CUDA_TRY(cudaMemcpy(base + parts[p_trees].off, trees.data(), trees.size() * sizeof(DevUrTree),
+                           cudaMemcpyHostToDevice),
+                "cudaMemcpy(trees)");
+  // the short scene form: one union_round tree, alone or beside one primitive
+  d.fast.kind = kFastNone;
+  if (im.fast_tree >= 0) {
+    d.fast.kind = kFastTree;
+    d.fast.tree = trees[im.leaves[im.fast_tree].first];
+    std::memcpy(d.fast.tmin, im.leaves[im.fast_tree].bmin, sizeof(d.fast.tmin));
+    std::memcpy(d.fast.tmax, im.leaves[im.fast_tree].bmax, sizeof(d.fast.tmax));
+    d.fast.prim = kNoPrim;
+    d.fast.tree_lhs = 1;
+    if (im.fast_prim >= 0) {
+      const ftgpu::HostLeaf& lf = im.leaves[im.fast_prim];
+      std::memcpy(d.fast.pmin, lf.bmin, sizeof(d.fast.pmin));
+      std::memcpy(d.fast.pmax, lf.bmax, sizeof(d.fast.pmax));
+      d.fast.prim = static_cast<uint32_t>(im.ur_prims.size()) | (im.cprims.back().leaf & ftd::kRareFlag);
+      d.fast.tree_lhs = im.bvh[im.bvh[im.bvh_root].lhs].leaf == im.fast_tree;
+    }
+  }
   // [0, 8): statistics counters; [8]: work-item counter of the persistent march
   FT_CUDA_TRY(cudaMalloc(&sc->d_stats, kStatWords * sizeof(unsigned long long)), "cudaMalloc(stats)");
   int sms = 0, per_sm = 0;
@@ -855,7 +970,7 @@ ft_status ft_scene_create(const ft_scene_desc* desc, ft_scene** out) {
   std::string err;
   bool built = false;
   try {
-    built = ftgpu::build_scene_image(*desc, &sc->img, &err);
+    built = ftgpu::build_scene_image(*desc, &sc->img, &err, false);
   } catch (...) {
     delete sc;
     throw;
@@ -892,7 +1007,7 @@ ft_status ft_scene_build_info(const ft_scene_desc* desc, ft_build_info* info) {
   ftgpu::SceneImage img;
   std::string err;
   auto t0 = std::chrono::steady_clock::now();
-  if (!ftgpu::build_scene_image(*desc, &img, &err)) return ftcommon::fail(FT_ERR_INVALID_ARGUMENT, err);
+  if (!ftgpu::build_scene_image(*desc, &img, &err, true)) return ftcommon::fail(FT_ERR_INVALID_ARGUMENT, err);
   auto t1 = std::chrono::steady_clock::now();
   std::memset(info, 0, sizeof(*info));
   info->leaves = static_cast<uint32_t>(img.leaves.size());
@@ -932,7 +1047,7 @@ ft_status ft_scene_last_launches(const ft_scene* sc, uint32_t* launches) {
 
 ft_status ft_scene_device_bytes(const ft_scene* sc, uint64_t* bytes) {
   if (!sc || !bytes) return ftcommon::fail(FT_ERR_INVALID_ARGUMENT, "scene and bytes must be non-null");
-  *bytes = sc->arena_bytes + sc->brick_bytes;
+  *bytes = sc->arena_bytes + sc->grid_bytes + sc->brick_bytes;
   return FT_OK;
 }
 
@@ -942,6 +1057,8 @@ void ft_scene_destroy(ft_scene* sc) {
   cudaGetDevice(&prev);
   cudaSetDevice(sc->device);
   cudaFree(sc->arena);
+  cudaFree(sc->grid_cells);
+  cudaFree(sc->grid_entries);
   cudaFree(sc->d_t);
   cudaFree(sc->d_mask);
   cudaFree(sc->d_mat);

@@ -549,7 +549,7 @@ __device__ __noinline__ void resolve_generic(const DevScene& S, int root, F3 p, 
     } else {
       GEntry r = st[--sp];
       GEntry l = st[--sp];
-      Info li{l.d, 0u, 0u}, ri{r.d, 0u, 0u};
+      Info li{l.d, ftd::kNoRef}, ri{r.d, ftd::kNoRef};
       float d = ftd::combine(n.kind, n.f[0], n.f[1], li, ri).d;
       bool diff;
       if (n.kind == FT_NODE_UNION) {
@@ -668,7 +668,7 @@ __device__ float ur_subtree_value(const DevScene& S, const DevUrTree& t, int c, 
     }
     float v = (F.v[0] == kInf && F.v[1] == kInf)
                   ? kInf
-                  : ftd::combine(FT_NODE_UNION_ROUND, t.r, 0.0f, Info{F.v[0], 0u, 0u}, Info{F.v[1], 0u, 0u}).d;
+                  : ftd::op_union_round(F.v[0], F.v[1], t.r);
     if (fp == 0) return v;
     --fp;
     fr[fp].v[fr[fp].stage - 1] = v;

@@ -149,7 +149,7 @@ __device__ __forceinline__ void wf_shade_job(const DevScene& S, const RayParams&
 
 // With kStats the kernel sums its work counters into stats[0 .. kNumCounters).
 template <bool kStats>
-__global__ void __launch_bounds__(128) wf_shade_kernel(DevScene S, RayParams P, const WJob* __restrict__ jobs,
+__global__ void __launch_bounds__(128) wf_shade_kernel(const __grid_constant__ DevScene S, const __grid_constant__ RayParams P, const WJob* __restrict__ jobs,
                                                        const unsigned long long* __restrict__ count,
                                                        unsigned long long cap, const WHit* __restrict__ hits,
                                                        WQueues Q, unsigned long long* __restrict__ stats) {
@@ -232,7 +232,8 @@ __device__ __noinline__ void wf_add_miss(const DevScene& S, const RayParams& P, 
 // (the launch is five per SM): on the 512-primitive field's depth-6 trace,
 // 181 ms of march per frame against 185 with six and 195 with four.
 template <bool kBatch, bool kStats>
-__global__ void __launch_bounds__(128, 5) wf_march_persistent(DevScene S0, RayParams P0, BatchView V,
+__global__ void __launch_bounds__(128, 5) wf_march_persistent(
+    const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ BatchView V,
                                                               const WJob* __restrict__ jobs,
                                                               const unsigned long long* __restrict__ count,
                                                               unsigned long long cap, WHit* __restrict__ hits,
@@ -328,8 +329,9 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(DevScene S0, RayPa
       h.t = hi;
       h.pos[0] = pos.x; h.pos[1] = pos.y; h.pos[2] = pos.z;
       h.normal[0] = nr.x; h.normal[1] = nr.y; h.normal[2] = nr.z;
-      h.mat = fin.mat;
-      h.obj = fin.obj;
+      const uint2 ids = surface_ids(S, fin.ref);
+      h.mat = ids.y;
+      h.obj = ids.x;
       hits[job] = h;
       live = false;
       continue;
@@ -369,46 +371,33 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(DevScene S0, RayPa
 }
 
 // A step of shadow_visibility (R:4706-4733): the leaf-box lower bound when it
-// exceeds max(8 eps, 0.02), else the exact distance.  With one or two leaves
-// the lower bound's box bounds are the ones the exact evaluation orders its
-// leaves by, so they are computed once; the values are those of
-// scene_lower_bound and scene_distance_inl.
+// exceeds max(8 eps, 0.02), else the exact distance.  The short scene form
+// computes its box bounds once for both.
 template <bool kStats>
 __device__ __forceinline__ float shadow_step_h(const DevScene& S, F3 p, float eps, Ctx<kStats>& cx) {
-  const DevBvhNode& root = S.bvh[S.bvh_root];
-  int leaf = root.leaf, second = -1;
-  float second_lb = kInf, lower;
-  bool small = true;
-  if (leaf >= 0) {
-    cx.box();
-    lower = node_lb(p, root.bmin, root.bmax);
-  } else {
-    const DevBvhNode& L = S.bvh[root.lhs];
-    const DevBvhNode& R = S.bvh[root.rhs];
-    if (L.leaf >= 0 && R.leaf >= 0) {
-      cx.box(3);
-      const float ll = node_lb(p, L.bmin, L.bmax), rl = node_lb(p, R.bmin, R.bmax);
-      lower = fminf(ll, rl);
-      const bool lfirst = ll <= rl;
-      leaf = lfirst ? L.leaf : R.leaf;
-      second = lfirst ? R.leaf : L.leaf;
-      second_lb = lfirst ? rl : ll;
-    } else {
-      small = false;
-      lower = scene_lower_bound(S, p, cx);
-    }
+  const DevFast& F = S.fast;
+  const float least = fmaxf(eps * 8.0f, 0.02f);
+  if (F.kind == kFastTree) {
+    const float t2 = ftd::aabb_lb2(p, F.tmin, F.tmax);
+    const bool alone = F.prim == kNoPrim;
+    const float p2 = alone ? kInf : ftd::aabb_lb2(p, F.pmin, F.pmax);
+    cx.box(alone ? 1 : 3);
+    const float lower = sqrtf(fminf(t2, p2));
+    if (lower > least) return lower;
+    cx.eval();
+    return fabsf(alone ? eval_urtree(S, F.tree, p, kInf, cx).d : tree_and_prim(S, p, t2, p2, cx).d);
   }
-  lower = fabsf(lower);
-  if (lower > fmaxf(eps * 8.0f, 0.02f)) return lower;
+  const float lower = fabsf(scene_lower_bound(S, p, cx));
+  if (lower > least) return lower;
   cx.eval();
-  return fabsf(small ? scene_distance_leaves<kStats, false>(S, p, leaf, second, second_lb, cx).d
-                     : scene_distance_bvh(S, p, cx).d);
+  return fabsf(scene_distance_general(S, p, cx).d);
 }
 
 // shadow_visibility (R:4706-4733) of every queued shadow job, one step per
 // iteration; the radiance gets contribution x visibility.
 template <bool kBatch, bool kStats>
-__global__ void __launch_bounds__(128, 8) wf_shadow_persistent(DevScene S0, RayParams P0, BatchView V,
+__global__ void __launch_bounds__(128, 8) wf_shadow_persistent(
+    const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ BatchView V,
                                                                const WShadow* __restrict__ shadows,
                                                                const unsigned long long* __restrict__ count,
                                                                unsigned long long cap, float* __restrict__ radiance,
@@ -482,7 +471,7 @@ __global__ void __launch_bounds__(128, 8) wf_shadow_persistent(DevScene S0, RayP
 // normal per sample; the hit record takes the point o + d t and the leaf
 // lookup there, as the wavefront march's final phase does, and a miss adds
 // the environment.
-__global__ void __launch_bounds__(128) wf_hits_from_depth_kernel(DevScene S, RayParams P,
+__global__ void __launch_bounds__(128) wf_hits_from_depth_kernel(const __grid_constant__ DevScene S, const __grid_constant__ RayParams P,
                                                                  const WJob* __restrict__ jobs, unsigned long long n,
                                                                  const float* __restrict__ t_in,
                                                                  const uint8_t* __restrict__ mask_in,
@@ -511,8 +500,9 @@ __global__ void __launch_bounds__(128) wf_hits_from_depth_kernel(DevScene S, Ray
     h.t = t;
     h.pos[0] = pos.x; h.pos[1] = pos.y; h.pos[2] = pos.z;
     h.normal[0] = normal_in[3 * s]; h.normal[1] = normal_in[3 * s + 1]; h.normal[2] = normal_in[3 * s + 2];
-    h.mat = fin.mat;
-    h.obj = fin.obj;
+    const uint2 ids = surface_ids(S, fin.ref);
+    h.mat = ids.y;
+    h.obj = ids.x;
     hits[i] = h;
   }
 }

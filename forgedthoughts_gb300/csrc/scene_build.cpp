@@ -55,7 +55,8 @@ float deg_to_rad(float d) { return d * (3.14159265358979323846f / 180.0f); }
 
 class Builder {
  public:
-  Builder(const ft_scene_desc& d, SceneImage* img, std::string* err) : d_(d), img_(img), err_(err) {}
+  Builder(const ft_scene_desc& d, SceneImage* img, std::string* err, bool lists)
+      : d_(d), img_(img), err_(err), lists_(lists) {}
 
   bool run() {
     if (!validate()) return false;
@@ -113,6 +114,17 @@ class Builder {
     img_->bvh_root = build_bvh(idx);
     for (size_t li = 0; li < img_->leaves.size(); ++li)
       if (!classify(li)) return false;
+    const auto& lv = img_->leaves;
+    for (int k = 0; lv.size() <= 2 && k < static_cast<int>(lv.size()); ++k) {
+      if (lv[k].kind != kLeafUrTree) continue;
+      if (lv.size() == 1) {
+        img_->fast_tree = k;
+      } else if (lv[1 - k].kind == kLeafPrim) {
+        img_->fast_tree = k;
+        img_->fast_prim = 1 - k;
+        img_->cprims.push_back(compact_prim(lv[1 - k].node, lv[1 - k]));
+      }
+    }
     return true;
   }
 
@@ -120,6 +132,7 @@ class Builder {
   const ft_scene_desc& d_;
   SceneImage* img_;
   std::string* err_;
+  bool lists_;
   std::vector<Box> bounds_;
   std::vector<char> have_bounds_;
 
@@ -585,7 +598,7 @@ class Builder {
     for (int a = 0; a < 3; ++a) dims[a] = std::max(1, static_cast<int>(std::ceil(ext[a] / cell)));
     if (static_cast<int64_t>(dims[0]) * dims[1] * dims[2] > 2 * 262144) return;
     int32_t first = 0;
-    if (!build_cells(t, g, all.mn, static_cast<float>(cell), dims, &first)) return;
+    if (lists_ && !build_cells(t, g, all.mn, static_cast<float>(cell), dims, &first)) return;
     t.cell = static_cast<float>(cell);
     t.inv_cell = 1.0f / t.cell;
     std::memcpy(t.gmin, all.mn, sizeof(t.gmin));
@@ -611,7 +624,7 @@ class Builder {
     int odims[3];
     for (int a = 0; a < 3; ++a) odims[a] = std::max(1, static_cast<int>(std::ceil(oext[a] / ocell)));
     if (static_cast<int64_t>(odims[0]) * odims[1] * odims[2] > 2 * (1 << 19)) return;
-    if (!build_cells(t, g, outer.mn, static_cast<float>(ocell), odims, &first)) return;
+    if (lists_ && !build_cells(t, g, outer.mn, static_cast<float>(ocell), odims, &first)) return;
     t.ocell = static_cast<float>(ocell);
     t.oinv_cell = 1.0f / t.ocell;
     std::memcpy(t.ogmin, outer.mn, sizeof(t.ogmin));
@@ -816,10 +829,46 @@ class Builder {
       for (uint32_t o : row_offsets[row]) img_->ur_cell_offsets.push_back(base + o);
       img_->ur_cell_prims.insert(img_->ur_cell_prims.end(), row_prims[row].begin(), row_prims[row].end());
       img_->ur_cell_gaps.insert(img_->ur_cell_gaps.end(), row_gaps[row].begin(), row_gaps[row].end());
-      for (int32_t pos : row_prims[row]) img_->ur_cell_nodes.push_back(img_->ur_prims[t.prim_first + pos]);
     }
     img_->ur_cell_offsets.push_back(static_cast<uint32_t>(img_->ur_cell_prims.size()));
     return true;
+  }
+
+  // Whether a primitive's distance is 1-Lipschitz and at least its box's: what
+  // the candidate grids and the box culling rest on.  The parser's shapes are;
+  // a node record may hold others (a rounding above the half size, a negative
+  // radius), which stay on the tree BVH.
+  bool sane_prim(const HostNode& n) const {
+    const float* f = n.f;
+    switch (n.kind) {
+      case FT_NODE_SPHERE: return f[0] >= 0.0f;
+      case FT_NODE_BOX:
+        return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[3] >= 0.0f && f[3] <= std::min(f[0], std::min(f[1], f[2]));
+      case FT_NODE_CYLINDER: return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[2] <= std::min(f[0], f[1]);
+      case FT_NODE_TORUS: return f[0] >= 0.0f && f[1] >= 0.0f;
+      default: return false;
+    }
+  }
+
+  CompactPrim compact_prim(int node, const HostLeaf& leaf) const {
+    const HostNode& n = img_->nodes[node];
+    CompactPrim c;
+    std::memset(&c, 0, sizeof(c));
+    std::memcpy(c.c, n.c, sizeof(c.c));
+    c.node = node;
+    c.leaf = static_cast<uint32_t>(&leaf - img_->leaves.data());
+    const bool y_only = !n.has_rot || (d_.nodes[node].rot_deg[0] == 0.0f && d_.nodes[node].rot_deg[2] == 0.0f);
+    if (!y_only || (n.kind != FT_NODE_SPHERE && n.kind != FT_NODE_BOX) || !sane_prim(n)) {
+      c.leaf |= 0x80000000u;
+      return c;
+    }
+    c.cos = n.has_rot ? n.cy : 1.0f;
+    c.sin = n.has_rot ? n.sy : 0.0f;
+    const float shell = n.kind == FT_NODE_SPHERE ? n.f[1] : n.f[4];
+    c.shell = shell > 0.0f ? shell : std::numeric_limits<float>::infinity();
+    c.rd = n.kind == FT_NODE_SPHERE ? n.f[0] : n.f[3];
+    for (int a = 0; a < 3; ++a) c.h[a] = n.kind == FT_NODE_SPHERE ? 0.0f : std::max(n.f[a] - n.f[3], 0.0f);
+    return c;
   }
 
   bool build_urtree(HostLeaf& leaf, float r, int depth) {
@@ -847,19 +896,21 @@ class Builder {
     };
     t.inner_root = walk(leaf.node);
     t.n_prims = static_cast<int32_t>(img_->ur_prims.size()) - t.prim_first;
-    // Parent links (the device folds one or two near primitives up to the
-    // root along them).
-    img_->ur_inner_up.resize(img_->ur_inner.size(), -1);
-    img_->ur_prim_up.resize(img_->ur_prims.size(), -1);
-    if (t.inner_root >= 0) {
-      for (size_t in = static_cast<size_t>(t.inner_root); in < img_->ur_inner.size(); ++in)
-        for (int side = 0; side < 2; ++side) {
-          int32_t c = img_->ur_inner[in].child[side];
-          int32_t link = static_cast<int32_t>(in << 1) | side;
-          if (c >= 0) img_->ur_inner_up[c] = link;
-          else img_->ur_prim_up[t.prim_first + (-c - 1)] = link;
-        }
-    }
+    // Compact records and root paths (the device folds near primitives along
+    // them).
+    for (int32_t i : std::vector<int32_t>(img_->ur_prims.begin() + t.prim_first, img_->ur_prims.end()))
+      img_->cprims.push_back(compact_prim(i, leaf));
+    img_->ur_paths.resize(img_->ur_prims.size(), UrPath{0, 0, 0});
+    std::function<void(int, uint64_t, uint32_t)> paths = [&](int c, uint64_t sides, uint32_t dep) {
+      if (c < 0) {
+        img_->ur_paths[t.prim_first + (-c - 1)] = UrPath{sides, dep, 0};
+        return;
+      }
+      const HostUrInner u = img_->ur_inner[c];
+      paths(u.child[0], sides, dep + 1);
+      paths(u.child[1], sides | (uint64_t(1) << dep), dep + 1);
+    };
+    if (t.inner_root >= 0) paths(t.inner_root, 0, 0);
     // Static material-model mixing of each inner node's primitives.
     img_->ur_inner_blend.resize(img_->ur_inner.size(), 0);
     for (size_t in = static_cast<size_t>(t.inner_root); in < img_->ur_inner.size(); ++in) {
@@ -876,7 +927,9 @@ class Builder {
     std::vector<int32_t> pos(t.n_prims);
     std::iota(pos.begin(), pos.end(), 0);
     t.bvh_root = build_ur_bvh(pos, 0, pos.size(), t.prim_first);
-    build_ur_grid(t);
+    bool sane = true;
+    for (int k = 0; k < t.n_prims; ++k) sane = sane && sane_prim(img_->nodes[img_->ur_prims[t.prim_first + k]]);
+    if (sane) build_ur_grid(t);
     if (!emit_program(leaf.node, &t.fallback_first, &t.fallback_count)) return false;
     leaf.kind = kLeafUrTree;
     leaf.first = static_cast<int32_t>(img_->urtrees.size());
@@ -903,9 +956,9 @@ class Builder {
 
 }  // namespace
 
-bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error) {
+bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error, bool lists) {
   *out = SceneImage{};
-  Builder b(desc, out, error);
+  Builder b(desc, out, error, lists);
   return b.run();
 }
 

@@ -38,6 +38,21 @@ struct HostBvhNode {  // leaf BVH in the reference's build order (R:693-732)
   int32_t lhs, rhs, leaf, pad;
 };
 
+struct CompactPrim {  // the device's three 16-byte words (compact_distance)
+  float c[3], cos;
+  float h[3], rd;
+  float sin, shell;
+  int32_t node;
+  uint32_t leaf;  // leaf index, high bit: not a compact kind, evaluated through its node
+};
+static_assert(sizeof(CompactPrim) == 48, "CompactPrim layout");
+
+struct UrPath {  // a tree primitive's way from the root: bit k is the side taken at depth k
+  uint64_t sides;
+  uint32_t depth;
+  uint32_t pad;
+};
+
 struct HostUrTree {
   float r;
   int32_t n_prims;
@@ -52,7 +67,6 @@ struct HostUrTree {
   float cell, inv_cell;
   int32_t dims[3];
   int32_t cell_first;  // into ur_cell_offsets (dims product + 1 entries)
-  int32_t pad;
   // Outer grid: coarser cells over a box around the first grid, for points
   // outside it (there every primitive is at least 2r away, so a cell lists
   // the primitives that can be the nearest).  odims[0] == 0: none.
@@ -60,7 +74,6 @@ struct HostUrTree {
   float ocell, oinv_cell;
   int32_t odims[3];
   int32_t ocell_first;
-  int32_t opad;
 };
 
 struct HostUrBvh {
@@ -90,13 +103,13 @@ struct SceneImage {
   // per ur_cell_prims entry: a lower bound of the distance from any point of
   // the cell to the primitive's box (the lists are sorted by it)
   std::vector<float> ur_cell_gaps;
-  // per ur_cell_prims entry: the primitive's node index (ur_prims of it), so
-  // the candidate walk loads it beside the position instead of after it
-  std::vector<int32_t> ur_cell_nodes;
-  // parent links of the union_round trees, (parent ur_inner index << 1) |
-  // side, -1 at the root: per ur_inner node and per primitive position
-  std::vector<int32_t> ur_inner_up;
-  std::vector<int32_t> ur_prim_up;
+  // A scene of one union_round tree, alone or beside one primitive: their
+  // leaves, -1 for other scenes (and no primitive).
+  int32_t fast_tree = -1, fast_prim = -1;
+  // compact records of the union_round trees' primitives, indexed as ur_prims,
+  // then that of fast_prim; root paths of the trees' primitives
+  std::vector<CompactPrim> cprims;
+  std::vector<UrPath> ur_paths;
   // per ur_inner node: 1 when its primitives use more than one material model
   // (blend_materials then yields a Blend whatever the weights)
   std::vector<int32_t> ur_inner_blend;
@@ -117,7 +130,10 @@ struct SceneImage {
 };
 
 // Build the image; returns false with `error` set on an invalid description.
-bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error);
+// With `lists` the candidate lists of the union_round grids are built here
+// (ft_scene_build_info reports them); without, only the grids' geometry: a
+// scene on a device builds its own lists there.
+bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error, bool lists);
 
 // Camera basis (R:6263-6286, render_api.rs:132-144) in f32.
 struct CameraBasis {
