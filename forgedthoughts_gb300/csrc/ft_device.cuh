@@ -177,13 +177,20 @@ FT_DEV float prim_distance(const DevNode& n, F3 p) { return prim_local(n.kind, n
 // every kernel rounds a distance alike, whatever the compiler contracts around
 // it, so that the depth march and the wavefront march take the same steps.
 // Other kinds set the rare flag and go through their node.
+//
+// kSphereYX: a sphere's squares are summed y first, as sphere_local does: a
+// hard union's spheres have always rounded that way, a union_round tree's
+// x first, and an ulp of a distance moves a silhouette pixel.
 constexpr uint32_t kRareFlag = 0x80000000u;
+template <bool kSphereYX>
 FT_DEV float compact_distance(float4 a, float4 b, float sn, float sh, F3 p) {
   const F3 t = f3(p.x - a.x, p.y - a.y, p.z - a.z);
   const float qx = fabsf(fmaf(a.w, t.x, sn * t.z)) - b.x, qy = fabsf(t.y) - b.y,
               qz = fabsf(fmaf(a.w, t.z, -sn * t.x)) - b.z;
   const float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
-  const float outside = sqrtf(fmaf(oz, oz, fmaf(ox, ox, oy * oy)));
+  const bool yx = kSphereYX && b.x == 0.0f;
+  const float u = yx ? oy : ox, v = yx ? ox : oy;
+  const float outside = sqrtf(fmaf(oz, oz, fmaf(u, u, v * v)));
   const float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);
   const float d = outside + inside - b.w;
   return rmax(d, -(d + sh));

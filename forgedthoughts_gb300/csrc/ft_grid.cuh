@@ -18,7 +18,9 @@
 // Blocks of 4^3 cells, one thread per cell.  The block first keeps the
 // primitives that pass the same test for the block as a whole (its cells'
 // centres and half diagonals lie inside the block's), so a cell tests a few
-// dozen primitives instead of all.  Two passes of the same kernel: the first
+// dozen primitives instead of all.  A hard union's walk gives up inside its
+// solids (see union_distance), so a cell that lies inside one primitive keeps
+// no list there.  Two passes of the same kernel: the first
 // counts a cell's entries, the second, with the memory in place, writes them.
 //
 // Bound by the distance evaluations of the block's primitives (a few million
@@ -35,6 +37,7 @@ struct GridJob {
   int32_t first;   // of the grid's cells
   int32_t prim_first, n_prims;
   float r, slack;
+  int32_t skip_inside;  // cells inside one primitive keep no list (kInsideCell)
 };
 
 constexpr int kGridBlockEdge = 4;
@@ -61,7 +64,7 @@ __device__ __noinline__ GridBound grid_bound(const DevScene& S, int i, F3 m, flo
     g.d = rare_distance(n, m);
   } else {
     radius = ftd::len3(f3(b.x, b.y, b.z)) + b.w;
-    g.d = ftd::compact_distance(a, b, e.x, e.y, m);
+    g.d = ftd::compact_distance<false>(a, b, e.x, e.y, m);
   }
   const float dx = fmaxf(fabsf(m.x - c.x) - half, 0.0f), dy = fmaxf(fabsf(m.y - c.y) - half, 0.0f),
               dz = fmaxf(fabsf(m.z - c.z) - half, 0.0f);
@@ -107,7 +110,7 @@ __global__ void __launch_bounds__(64) grid_cells_kernel(const __grid_constant__ 
   const bool all = n_keep > kGridKeep;
   const int n = all ? J.n_prims : n_keep;
   const int x = b0[0] + (t & 3), y = b0[1] + (t >> 2 & 3), z = b0[2] + (t >> 4);
-  const bool mine = x < J.dims[0] && y < J.dims[1] && z < J.dims[2];
+  bool mine = x < J.dims[0] && y < J.dims[1] && z < J.dims[2];
   const int cell = J.first + x + J.dims[0] * (y + J.dims[1] * z);
   const float half = 0.5f * J.cell + pad;
   const F3 m = f3(J.gmin[0] + (x + 0.5f) * J.cell, J.gmin[1] + (y + 0.5f) * J.cell, J.gmin[2] + (z + 0.5f) * J.cell);
@@ -119,10 +122,15 @@ __global__ void __launch_bounds__(64) grid_cells_kernel(const __grid_constant__ 
     limit = fmaxf(J.r, best + half * 1.7320509f) + J.slack;
     if (kFill) {
       count = cells[cell].y;
+      if (count == kInsideCell) {
+        count = 0;
+        mine = false;
+      }
     } else {
-      for (int k = 0; k < n; ++k)
+      const bool inside = J.skip_inside && best + half * 1.7320509f < -J.slack;
+      for (int k = 0; k < (inside ? 0 : n); ++k)
         count += grid_bound(S, J.prim_first + (all ? k : keep[k]), m, half).low - J.slack < limit;
-      cells[cell] = make_uint2(0u, count);
+      cells[cell] = make_uint2(0u, inside ? kInsideCell : count);
     }
   }
   // the block's entries: counted into the total, or allocated from it
@@ -140,35 +148,23 @@ __global__ void __launch_bounds__(64) grid_cells_kernel(const __grid_constant__ 
   if (!mine) return;
   const unsigned at = static_cast<unsigned>(base) + scan - count;
   cells[cell] = make_uint2(at, count);
-  // Ascending by (bound, index): short lists by repeated selection, which
-  // writes each entry once; long ones are written and heap sorted in place.
-  auto entry = [&](int k, uint2* out) {
+  // Ascending by (bound, index): a short list by insertion as it is written, a
+  // long one by heap sort in place.
+  auto before = [](uint2 u, uint2 v) { return u.x < v.x || (u.x == v.x && (u.y & ~ftd::kRareFlag) < (v.y & ~ftd::kRareFlag)); };
+  uint2* list = entries + at;
+  const bool insert = count <= 24;
+  unsigned w = 0;
+  for (int k = 0; k < n && w < count; ++k) {
     const int i = J.prim_first + (all ? k : keep[k]);
     const GridBound g = grid_bound(S, i, m, half);
     const float low = g.low - J.slack;
-    *out = make_uint2(__float_as_uint(fmaxf(low, 0.0f)), static_cast<uint32_t>(i) | g.rare);
-    return low < limit;
-  };
-  auto before = [](uint2 u, uint2 v) { return u.x < v.x || (u.x == v.x && (u.y & ~ftd::kRareFlag) < (v.y & ~ftd::kRareFlag)); };
-  uint2* list = entries + at;
-  if (count <= 32) {
-    uint2 last = make_uint2(0u, 0u);
-    for (unsigned j = 0; j < count; ++j) {
-      uint2 next = make_uint2(0xffffffffu, 0xffffffffu);
-      for (int k = 0; k < n; ++k) {
-        uint2 u;
-        if (entry(k, &u) && (j == 0 || before(last, u)) && before(u, next)) next = u;
-      }
-      if (next.x == 0xffffffffu) break;  // (not reached: both passes find the same entries)
-      list[j] = last = next;
-    }
-    return;
+    if (!(low < limit)) continue;
+    const uint2 u = make_uint2(__float_as_uint(fmaxf(low, 0.0f)), static_cast<uint32_t>(i) | g.rare);
+    unsigned j = w++;
+    for (; insert && j > 0 && before(u, list[j - 1]); --j) list[j] = list[j - 1];
+    list[j] = u;
   }
-  unsigned w = 0;
-  for (int k = 0; k < n && w < count; ++k) {
-    uint2 u;
-    if (entry(k, &u)) list[w++] = u;
-  }
+  if (insert) return;
   auto sift = [&](unsigned root, unsigned end) {
     const uint2 v = list[root];
     for (unsigned child = 2 * root + 1; child < end; child = 2 * root + 1) {

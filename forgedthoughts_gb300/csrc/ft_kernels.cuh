@@ -38,7 +38,7 @@ struct DevBvhNode {
 // Candidate grid: cell c of the box from gmin lists (DevScene::cells, cell
 // first + c) the primitives that can be the nearest or lie within the blend
 // radius at some point of it.  dims[0] == 0: none.
-struct DevGrid {
+struct alignas(16) DevGrid {
   float gmin[3];
   float inv_cell;
   int32_t dims[3];
@@ -47,6 +47,7 @@ struct DevGrid {
 struct DevUrTree {
   float r;
   int32_t n_prims, prim_first, bvh_root, inner_root, depth, fallback_first, fallback_count;
+  int32_t far_first, far_end;  // far-walk nodes
   DevGrid fine, outer;
 };
 struct DevUrBvh {
@@ -59,18 +60,26 @@ struct DevUrInner {
 };
 
 // Scenes whose distance has a short form, taken by the march loops without
-// the general leaf walk.  kFastTree: one union_round tree, alone or beside one
-// primitive (a ground); the copies of the tree's header and the leaf boxes are
-// kernel parameters, read from the constant bank.
-enum FastKind : int32_t { kFastNone = 0, kFastTree = 1 };
-struct DevFast {
+// the general leaf walk; its data are kernel parameters, read from the constant
+// bank.
+//   kFastTree   one union_round tree (`tree`, box 1), alone or beside one
+//               primitive (entry[0], box 0);
+//   kFastPair   two primitives (entry and boxes 0, 1: the BVH root's children);
+//   kFastUnion  primitives only: the first n_always compact records at every
+//               point, the others through the candidate grids and far walk of
+//               `tree`, box 1 around them.
+enum FastKind : int32_t { kFastNone = 0, kFastTree = 1, kFastPair = 2, kFastUnion = 3 };
+struct alignas(16) DevFast {
   int32_t kind;
-  uint32_t prim;       // kFastTree: the primitive leaf's compact entry, kNoPrim for a tree alone
-  int32_t tree_lhs;    // the tree is the BVH root's left child
-  float pmin[3], pmax[3], tmin[3], tmax[3];
+  int32_t n_always;
+  int32_t tree_lhs;   // kFastTree: the tree is the BVH root's left child
+  int32_t all;        // kFastUnion: every primitive is in the first n_always
+  uint32_t entry[2];  // compact entries, kNoPrim for none
+  float bmin[2][3], bmax[2][3];
   DevUrTree tree;
 };
 constexpr uint32_t kNoPrim = 0xffffffffu;
+constexpr uint32_t kInsideCell = 0xffffffffu;  // entry count of a cell inside one primitive
 
 struct DevScene {
   DevFast fast;
@@ -86,6 +95,8 @@ struct DevScene {
   const float4* __restrict__ cprims;   // compact primitives (three words each, compact_distance)
   const uint4* __restrict__ ur_paths;  // per tree primitive: sides taken from the root (low, high word), depth
   const uint2* __restrict__ cells;     // per grid cell: first entry, entries
+  const float4* __restrict__ far_nodes;     // two words per node (ftgpu::FarNode)
+  const uint32_t* __restrict__ far_entries;  // compact entries of the far walks' leaves
   const uint2* __restrict__ entries;   // lower bound of the distance from the cell (ascending), compact index | rare
   const ft_program* __restrict__ programs;
   const ft_instr* __restrict__ instrs;
@@ -331,13 +342,13 @@ __device__ __noinline__ Info eval_generic(const DevScene& S, int first, int coun
 // where their paths first differ, and no node is loaded on the way.
 
 // Primitive `idx` of the compact array at p.
-template <bool kStats>
+template <bool kSphereYX = false, bool kStats>
 __device__ __forceinline__ float compact_at(const DevScene& S, uint32_t entry, F3 p, Ctx<kStats>& cx) {
   cx.prim();
   const float4* w = S.cprims + 3 * static_cast<size_t>(entry & ~ftd::kRareFlag);
   const float4 c = __ldg(w + 2);
   if (entry & ftd::kRareFlag) return rare_distance(S.nodes[__float_as_int(c.z)], p);
-  return ftd::compact_distance(__ldg(w), __ldg(w + 1), c.x, c.y, p);
+  return ftd::compact_distance<kSphereYX>(__ldg(w), __ldg(w + 1), c.x, c.y, p);
 }
 
 // Value one level up of a subtree whose sibling holds no near primitive: the
@@ -472,8 +483,44 @@ __device__ __forceinline__ Info ur_value(const DevScene& S, const DevUrTree& t, 
   return ur_fold_many(S, t.r, idx, dist, n.nn, cx);
 }
 
-// Points outside both candidate grids walk the tree's BVH, out of line: it is
-// rare beside the grids' cell walks, whose code stays in the march loops.
+// Nearest primitive below best.d from a point outside the candidate grids,
+// where every primitive is outside its box: the nodes in depth-first order, a
+// subtree skipped when its box is not nearer than the best so far.  Out of
+// line: it is rare beside the grids' cell walks, whose code stays in the march
+// loops.  A node is two 16-byte loads and there is no stack: the leaf-BVH walk
+// it replaces for these points spent over a thousand cycles on a node (14
+// scalar loads and a stack in local memory), and rays that pass over a scene
+// set the time of a small frame.  `tie`: whether the distance found occurred
+// twice.
+template <bool kSphereYX, bool kStats>
+__device__ __noinline__ Info far_nearest(const DevScene& S, const DevUrTree& t, F3 p, Info best, bool* tie,
+                                         Ctx<kStats>& cx) {
+  bool same = false;
+  for (int k = t.far_first; k < t.far_end;) {
+    const float4 a = __ldg(S.far_nodes + 2 * static_cast<size_t>(k));
+    const float4 b = __ldg(S.far_nodes + 2 * static_cast<size_t>(k) + 1);
+    const float mn[3] = {a.x, a.y, a.z}, mx[3] = {b.x, b.y, b.z};
+    cx.box();
+    if (ftd::aabb_lb2(p, mn, mx) >= best.d * best.d) {
+      k = __float_as_int(a.w);
+      continue;
+    }
+    const int prims = __float_as_int(b.w);
+    if (prims >= 0) {
+      for (int e = prims >> 3, end = e + (prims & 7); e < end; ++e) {
+        const uint32_t entry = __ldg(S.far_entries + e);
+        const float d = compact_at<kSphereYX>(S, entry, p, cx);
+        same = d == best.d || (same && !(d < best.d));
+        if (d < best.d) best = Info{d, ~static_cast<int32_t>(entry & ~ftd::kRareFlag)};
+      }
+    }
+    ++k;
+  }
+  *tie = same;
+  return best;
+}
+
+// The BVH walk of a tree without candidate grids, out of line.
 template <bool kStats>
 __device__ __noinline__ Info eval_urtree_far(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
                                              Ctx<kStats>& cx) {
@@ -535,13 +582,17 @@ __device__ __forceinline__ bool grid_cell(const DevGrid& g, F3 p, int* cell) {
 // The tree's value at p, exact where it is below `cutoff`: the candidates of
 // p's cell in the fine grid, or outside it in the coarser outer grid around it
 // (its cells list the primitives that can be the nearest there), else the
-// tree's BVH.  A cell's list is sorted by a lower bound of its points'
+// nearest primitive (outside the grids all are more than r away).  A cell's list is sorted by a lower bound of its points'
 // distances, so the first entry at or above the running limit ends it.
 template <bool kStats>
 __device__ __forceinline__ Info eval_urtree(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
                                             Ctx<kStats>& cx) {
   int cell = 0;
-  if (!grid_cell(t.fine, p, &cell) && !grid_cell(t.outer, p, &cell)) return eval_urtree_far(S, t, p, cutoff, cx);
+  if (!grid_cell(t.fine, p, &cell) && !grid_cell(t.outer, p, &cell)) {
+    bool tie;
+    return t.fine.dims[0] > 0 ? far_nearest<false>(S, t, p, Info{cutoff, ftd::kNoRef}, &tie, cx)
+                              : eval_urtree_far(S, t, p, cutoff, cx);
+  }
   const uint2 range = __ldg(S.cells + cell);
   const float r = t.r;
   UrNear n;
@@ -663,6 +714,8 @@ __device__ __noinline__ Info scene_distance_general(const DevScene& S, F3 p, Ctx
   return scene_distance_leaves(S, p, leaf, second, second_lb, cx);
 }
 
+__device__ __forceinline__ int32_t compact_ref(uint32_t entry) { return ~static_cast<int32_t>(entry & ~ftd::kRareFlag); }
+
 // kFastTree with a primitive leaf: the two-leaf walk above (nearer box first,
 // the other leaf when its box bound is not above the distance found) with the
 // primitive evaluated first in either order, so that its distance bounds the
@@ -674,11 +727,81 @@ template <bool kStats>
 __device__ __forceinline__ Info tree_and_prim(const DevScene& S, F3 p, float t2, float p2, Ctx<kStats>& cx) {
   const DevFast& F = S.fast;
   const bool tree_first = F.tree_lhs ? t2 <= p2 : t2 < p2;
-  const Info prim{compact_at(S, F.prim, p, cx), ~static_cast<int32_t>(F.prim & ~ftd::kRareFlag)};
+  const Info prim{compact_at(S, F.entry[0], p, cx), compact_ref(F.entry[0])};
   if (!tree_first && !(sqrtf(t2) <= prim.d)) return prim;
   const Info tree = eval_urtree(S, F.tree, p, tree_first && prim.d < 0.0f ? kInf : prim.d, cx);
   if (!tree_first) return tree.d < prim.d ? tree : prim;
   return prim.d < tree.d && sqrtf(p2) <= tree.d ? prim : tree;
+}
+
+// kFastPair: the two-leaf walk of two primitives.
+template <bool kStats>
+__device__ __forceinline__ Info pair_distance(const DevScene& S, F3 p, float l2, float r2, Ctx<kStats>& cx) {
+  const DevFast& F = S.fast;
+  const bool lfirst = l2 <= r2;
+  const uint32_t e0 = lfirst ? F.entry[0] : F.entry[1], e1 = lfirst ? F.entry[1] : F.entry[0];
+  const Info a{compact_at<true>(S, e0, p, cx), compact_ref(e0)};
+  if (!(sqrtf(lfirst ? r2 : l2) <= a.d)) return a;
+  const Info b{compact_at<true>(S, e1, p, cx), compact_ref(e1)};
+  return b.d < a.d ? b : a;
+}
+
+// kFastUnion: the nearest of the always-evaluated primitives (all of a small
+// scene; else the few whose box dwarfs the rest, a ground) and of the
+// candidates of p's cell, in ascending order of their lower bounds, up to the
+// first that cannot be nearer.
+//
+// The leaf-BVH walk (bvh_distance_info) gives the same nearest distance with
+// two exceptions that depend on its order: inside the solids it keeps the
+// first negative distance found (every other box bound is at least 0), and of
+// equal distances the first.  So a point with two negative distances, or with
+// a tie for the nearest, takes that walk, and one in a cell inside a solid.  A
+// point outside both grids takes the far walk unless the box of the listed
+// primitives is no nearer than the distance found.
+template <bool kStats>
+__device__ __forceinline__ Info union_distance(const DevScene& S, F3 p, Ctx<kStats>& cx) {
+  const DevFast& F = S.fast;
+  Info best{kInf, ftd::kNoRef};
+  int negative = 0;
+  bool tie = false;
+  auto add = [&](float d, int i) {
+    tie = d == best.d || (tie && !(d < best.d));
+    if (d < best.d) best = Info{d, ~i};
+    negative += d < 0.0f;
+  };
+#pragma unroll 4
+  for (int i = 0; i < F.n_always; ++i) {  // the same record for every lane
+    const float4* w = S.cprims + 3 * i;
+    const float4 a = __ldg(w), b = __ldg(w + 1), c = __ldg(w + 2);
+    cx.prim();
+    add(__float_as_uint(c.w) & ftd::kRareFlag ? rare_distance(S.nodes[__float_as_int(c.z)], p)
+                                              : ftd::compact_distance<true>(a, b, c.x, c.y, p),
+        i);
+  }
+  bool walk = false;  // take the leaf-BVH walk
+  if (!F.all) {
+    int cell = 0;
+    if (grid_cell(F.tree.fine, p, &cell) || grid_cell(F.tree.outer, p, &cell)) {
+      const uint2 range = __ldg(S.cells + cell);
+      walk = range.y == kInsideCell;
+      for (uint32_t k = range.x, end = walk ? k : range.x + range.y; k < end; ++k) {
+        const uint2 e = __ldg(S.entries + k);
+        cx.cand();
+        if (__uint_as_float(e.x) >= fmaxf(best.d, 1.17549435e-38f)) break;
+        add(compact_at<true>(S, e.y, p, cx), static_cast<int>(e.y & ~ftd::kRareFlag));
+      }
+    } else {
+      cx.box();
+      if (sqrtf(ftd::aabb_lb2(p, F.bmin[1], F.bmax[1])) < best.d) {
+        bool same;
+        const Info far = far_nearest<true>(S, F.tree, p, best, &same, cx);
+        tie = same || (tie && far.ref == best.ref);
+        best = far;
+      }
+    }
+  }
+  if (walk || tie || negative > 1) return scene_distance_bvh(S, p, cx);
+  return best;
 }
 
 // The scene distance at p (Accelerator::distance_info): the short form of the
@@ -688,10 +811,12 @@ template <bool kStats>
 __device__ __forceinline__ Info scene_distance_inl(const DevScene& S, F3 p, Ctx<kStats>& cx) {
   cx.eval();
   const DevFast& F = S.fast;
-  if (F.kind != kFastTree) return scene_distance_general(S, p, cx);
-  if (F.prim == kNoPrim) return eval_urtree(S, F.tree, p, kInf, cx);
+  if (F.kind == kFastUnion) return union_distance(S, p, cx);
+  if (F.kind == kFastNone) return scene_distance_general(S, p, cx);
+  if (F.entry[0] == kNoPrim) return eval_urtree(S, F.tree, p, kInf, cx);
   cx.box(2);
-  return tree_and_prim(S, p, ftd::aabb_lb2(p, F.tmin, F.tmax), ftd::aabb_lb2(p, F.pmin, F.pmax), cx);
+  const float l2 = ftd::aabb_lb2(p, F.bmin[0], F.bmax[0]), r2 = ftd::aabb_lb2(p, F.bmin[1], F.bmax[1]);
+  return F.kind == kFastTree ? tree_and_prim(S, p, r2, l2, cx) : pair_distance(S, p, l2, r2, cx);
 }
 
 template <bool kStats>
@@ -968,7 +1093,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(
 #ifdef FT_JIT
   constexpr bool kRayYFirst = true;
 #else
-  constexpr bool kRayYFirst = kBricks && !kBatch;
+  constexpr bool kRayYFirst = kBricks;
 #endif
   const unsigned lane = threadIdx.x & 31u;
   const bool want_normal = normal_out != nullptr;

@@ -34,6 +34,7 @@ static_assert(sizeof(DevLeaf) == sizeof(ftgpu::HostLeaf), "leaf layout");
 static_assert(sizeof(DevBvhNode) == sizeof(ftgpu::HostBvhNode), "bvh layout");
 static_assert(3 * sizeof(float4) == sizeof(ftgpu::CompactPrim), "compact primitive layout");
 static_assert(sizeof(uint4) == sizeof(ftgpu::UrPath), "root path layout");
+static_assert(2 * sizeof(float4) == sizeof(ftgpu::FarNode), "far node layout");
 static_assert(sizeof(DevUrBvh) == sizeof(ftgpu::HostUrBvh), "urbvh layout");
 static_assert(sizeof(DevUrInner) == sizeof(ftgpu::HostUrInner), "urinner layout");
 
@@ -185,6 +186,41 @@ void prof_collect(ft_scene* sc) {
   sc->prof_pending.clear();
 }
 
+float aabb_volume(const float* mn, const float* mx) {
+  float v = 1.0f;
+  for (int a = 0; a < 3; ++a) v *= std::max(mx[a] - mn[a], 1.0e-6f);
+  return v;
+}
+
+// Leaves evaluated exactly at every far-field step instead of being cached:
+// the few whose box dwarfs the box of all remaining leaves (a ground slab).
+std::vector<int> choose_exact_leaves(const ftgpu::SceneImage& im) {
+  const int n = static_cast<int>(im.leaves.size());
+  std::vector<int> order(n);
+  for (int i = 0; i < n; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return aabb_volume(im.leaves[a].bmin, im.leaves[a].bmax) > aabb_volume(im.leaves[b].bmin, im.leaves[b].bmax);
+  });
+  std::vector<int> exact;
+  std::vector<char> is_exact(n, 0);
+  for (int k = 0; k < n - 1 && static_cast<int>(exact.size()) < kMaxExactLeaves; ++k) {
+    int i = order[k];
+    float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
+    for (int j = 0; j < n; ++j) {
+      if (j == i || is_exact[j]) continue;
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = std::min(mn[a], im.leaves[j].bmin[a]);
+        mx[a] = std::max(mx[a], im.leaves[j].bmax[a]);
+      }
+    }
+    if (aabb_volume(im.leaves[i].bmin, im.leaves[i].bmax) <= 8.0f * aabb_volume(mn, mx)) break;
+    exact.push_back(i);
+    is_exact[i] = 1;
+  }
+  return exact;
+}
+
+
 // Candidate-list entries of all grids of a scene (8 bytes each); a grid past
 // it is dropped, and its points take the tree BVH.
 constexpr uint64_t kMaxGridEntries = uint64_t(1) << 26;
@@ -260,6 +296,35 @@ DevGrid dev_grid(const GridJob& j) {
   return g;
 }
 
+// Most leaves of a hard union that are all evaluated at every point.
+constexpr size_t kBruteLeaves = 4;
+
+// Grids of a hard union's listed primitives, whose boxes fill mn..mx: a fine
+// one over that box widened by a tenth, and a coarser one half an extent wider
+// around it.  Both end on their own entry caps.
+void union_grids(const float mn[3], const float mx[3], int32_t first, int32_t n, std::vector<GridJob>* jobs) {
+  const float widest = std::max({mx[0] - mn[0], mx[1] - mn[1], mx[2] - mn[2]});
+  for (int k = 0; k < 2; ++k) {
+    const float widen = (k == 0 ? 0.05f : 0.6f) * widest;
+    const double target = k == 0 ? std::min(131072.0, std::max(4096.0, 128.0 * n)) : std::min(65536.0, std::max(4096.0, 32.0 * n));
+    float gmin[3];
+    double volume = 1.0, ext[3];
+    for (int a = 0; a < 3; ++a) {
+      gmin[a] = mn[a] - widen;
+      ext[a] = static_cast<double>(mx[a] - mn[a]) + 2.0 * widen;
+      volume *= ext[a];
+    }
+    const double cell = std::cbrt(volume / target);
+    if (!(cell > 0.0) || !std::isfinite(cell)) return;
+    int32_t dims[3];
+    for (int a = 0; a < 3; ++a) dims[a] = std::max(1, static_cast<int32_t>(std::ceil(ext[a] / cell)));
+    if (static_cast<int64_t>(dims[0]) * dims[1] * dims[2] > 4 * 131072) return;
+    GridJob j = grid_job(gmin, static_cast<float>(cell), dims, first, n, 1.17549435e-38f);
+    j.skip_inside = 1;
+    jobs->push_back(j);
+  }
+}
+
 ft_status upload_scene(ft_scene* sc) {
   const ftgpu::SceneImage& im = sc->img;
   struct Part {
@@ -268,6 +333,8 @@ ft_status upload_scene(ft_scene* sc) {
     size_t off;
   };
   std::vector<DevUrTree> trees;
+  std::vector<ftgpu::FarNode> far_nodes;
+  std::vector<uint32_t> far_entries;
   for (const ftgpu::HostUrTree& t : im.urtrees) {
     DevUrTree d{};
     d.r = t.r;
@@ -278,8 +345,37 @@ ft_status upload_scene(ft_scene* sc) {
     d.depth = t.depth;
     d.fallback_first = t.fallback_first;
     d.fallback_count = t.fallback_count;
+    d.far_first = static_cast<int32_t>(far_nodes.size());
+    ftgpu::build_far_tree(im, im.cprims, t.prim_first, t.n_prims, &far_nodes, &far_entries);
+    d.far_end = static_cast<int32_t>(far_nodes.size());
     trees.push_back(d);
   }
+  // A hard union's records: the primitives evaluated at every point first (all
+  // of up to kBruteLeaves: their loads are the same for every lane and do not
+  // depend on one another; else the few that dwarf the rest), the listed after.
+  std::vector<ftgpu::CompactPrim> cprims = im.cprims;
+  int32_t n_always = 0, n_listed = 0;
+  if (im.fast_union && im.leaves.size() != 2) {
+    n_always = static_cast<int32_t>(im.leaves.size());
+    if (im.leaves.size() > kBruteLeaves) {
+      std::vector<char> always(im.leaves.size(), 0);
+      for (int k : choose_exact_leaves(im)) always[k] = 1;
+      std::stable_partition(cprims.begin(), cprims.end(),
+                            [&](const ftgpu::CompactPrim& c) { return always[c.leaf & ~ftd::kRareFlag] != 0; });
+      n_always = static_cast<int32_t>(std::count(always.begin(), always.end(), 1));
+      n_listed = static_cast<int32_t>(im.leaves.size()) - n_always;
+    }
+  }
+  ftgpu::build_far_tree(im, cprims, n_always, n_listed, &far_nodes, &far_entries);  // (a union has no trees before it)
+  auto listed_box = [&](float mn[3], float mx[3]) {
+    for (int k = n_always; k < n_always + n_listed; ++k) {
+      const ftgpu::HostLeaf& lf = im.leaves[cprims[k].leaf & ~ftd::kRareFlag];
+      for (int a = 0; a < 3; ++a) {
+        mn[a] = std::min(mn[a], lf.bmin[a]);
+        mx[a] = std::max(mx[a], lf.bmax[a]);
+      }
+    }
+  };
   std::vector<Part> parts;
   auto part = [&](const void* src, size_t bytes) {
     parts.push_back(Part{src, bytes, 0});
@@ -289,9 +385,10 @@ ft_status upload_scene(ft_scene* sc) {
   const size_t p_nodes = vec(im.nodes), p_leaves = vec(im.leaves), p_bvh = vec(im.bvh), p_gops = vec(im.gops),
                p_trees = vec(trees), p_ur_bvh = vec(im.ur_bvh), p_ur_bvh_prims = vec(im.ur_bvh_prims),
                p_ur_prims = vec(im.ur_prims), p_ur_inner = vec(im.ur_inner), p_programs = vec(im.programs),
-               p_instrs = vec(im.instrs), p_cprims = vec(im.cprims), p_paths = vec(im.ur_paths),
+               p_instrs = vec(im.instrs), p_cprims = vec(cprims), p_paths = vec(im.ur_paths),
                p_materials = vec(im.materials), p_lights = vec(im.lights), p_op_begin = vec(im.node_op_begin),
-               p_op_end = vec(im.node_op_end), p_blend = vec(im.ur_inner_blend), p_obj = vec(im.obj_node);
+               p_op_end = vec(im.node_op_end), p_blend = vec(im.ur_inner_blend), p_obj = vec(im.obj_node),
+               p_far = vec(far_nodes), p_far_entries = vec(far_entries);
   size_t total = 0;
   for (Part& p : parts) {
     p.off = total;
@@ -327,6 +424,8 @@ ft_status upload_scene(ft_scene* sc) {
   at(p_op_end, d.node_op_end);
   at(p_blend, d.ur_inner_blend);
   at(p_obj, d.obj_node);
+  at(p_far, d.far_nodes);
+  at(p_far_entries, d.far_entries);
   d.n_obj_node = static_cast<int32_t>(im.obj_node.size());
   d.n_materials = static_cast<int32_t>(im.materials.size());
   d.n_lights = static_cast<int32_t>(im.lights.size());
@@ -334,9 +433,15 @@ ft_status upload_scene(ft_scene* sc) {
   d.bvh_root = im.bvh_root;
   std::memcpy(d.smin, im.scene_min, sizeof(d.smin));
   std::memcpy(d.smax, im.scene_max, sizeof(d.smax));
-  // the union_round trees' candidate grids (fine, outer)
+  // the union_round trees' candidate grids (fine, outer), or those of a hard
+  // union's listed primitives
   std::vector<GridJob> jobs;
   std::vector<std::pair<size_t, bool>> owner;
+  if (n_listed > 0) {
+    float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
+    listed_box(mn, mx);
+    union_grids(mn, mx, n_always, n_listed, &jobs);
+  }
   for (size_t k = 0; k < im.urtrees.size(); ++k) {
     const ftgpu::HostUrTree& t = im.urtrees[k];
     if (t.dims[0] <= 0) continue;
@@ -347,27 +452,47 @@ ft_status upload_scene(ft_scene* sc) {
     owner.emplace_back(k, true);
   }
   if (ft_status s = build_grids(sc, &jobs)) return s;
-  for (size_t k = 0; k < jobs.size(); ++k)
+  for (size_t k = 0; k < owner.size(); ++k)
     (owner[k].second ? trees[owner[k].first].outer : trees[owner[k].first].fine) = dev_grid(jobs[k]);
   if (!trees.empty())
     FT_CUDA_TRY(cudaMemcpy(base + parts[p_trees].off, trees.data(), trees.size() * sizeof(DevUrTree),
                            cudaMemcpyHostToDevice),
                 "cudaMemcpy(trees)");
-  // the short scene form: one union_round tree, alone or beside one primitive
-  d.fast.kind = kFastNone;
+  // the short scene form, if the scene has one
+  DevFast& F = d.fast;
+  F.kind = kFastNone;
+  F.entry[0] = F.entry[1] = kNoPrim;
+  auto box = [&](int k, const float* mn, const float* mx) {
+    std::memcpy(F.bmin[k], mn, sizeof(F.bmin[k]));
+    std::memcpy(F.bmax[k], mx, sizeof(F.bmax[k]));
+  };
   if (im.fast_tree >= 0) {
-    d.fast.kind = kFastTree;
-    d.fast.tree = trees[im.leaves[im.fast_tree].first];
-    std::memcpy(d.fast.tmin, im.leaves[im.fast_tree].bmin, sizeof(d.fast.tmin));
-    std::memcpy(d.fast.tmax, im.leaves[im.fast_tree].bmax, sizeof(d.fast.tmax));
-    d.fast.prim = kNoPrim;
-    d.fast.tree_lhs = 1;
+    F.kind = kFastTree;
+    F.tree = trees[im.leaves[im.fast_tree].first];
+    F.tree_lhs = 1;
+    box(1, im.leaves[im.fast_tree].bmin, im.leaves[im.fast_tree].bmax);
     if (im.fast_prim >= 0) {
-      const ftgpu::HostLeaf& lf = im.leaves[im.fast_prim];
-      std::memcpy(d.fast.pmin, lf.bmin, sizeof(d.fast.pmin));
-      std::memcpy(d.fast.pmax, lf.bmax, sizeof(d.fast.pmax));
-      d.fast.prim = static_cast<uint32_t>(im.ur_prims.size()) | (im.cprims.back().leaf & ftd::kRareFlag);
-      d.fast.tree_lhs = im.bvh[im.bvh[im.bvh_root].lhs].leaf == im.fast_tree;
+      box(0, im.leaves[im.fast_prim].bmin, im.leaves[im.fast_prim].bmax);
+      F.entry[0] = static_cast<uint32_t>(im.ur_prims.size()) | (cprims.back().leaf & ftd::kRareFlag);
+      F.tree_lhs = im.bvh[im.bvh[im.bvh_root].lhs].leaf == im.fast_tree;
+    }
+  } else if (im.fast_union && im.leaves.size() == 2) {
+    F.kind = kFastPair;
+    for (int k = 0; k < 2; ++k) {
+      const int leaf = im.bvh[k == 0 ? im.bvh[im.bvh_root].lhs : im.bvh[im.bvh_root].rhs].leaf;
+      F.entry[k] = static_cast<uint32_t>(leaf) | (cprims[leaf].leaf & ftd::kRareFlag);
+      box(k, im.leaves[leaf].bmin, im.leaves[leaf].bmax);
+    }
+  } else if (im.fast_union) {
+    F.kind = kFastUnion;
+    F.n_always = n_always;
+    F.all = n_listed == 0;
+    if (n_listed > 0) {
+      float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
+      listed_box(mn, mx);
+      box(1, mn, mx);
+      F.tree.far_end = static_cast<int32_t>(far_nodes.size());
+      for (size_t k = 0; k < jobs.size(); ++k) (k == 0 ? F.tree.fine : F.tree.outer) = dev_grid(jobs[k]);
     }
   }
   // [0, 8): statistics counters; [8]: work-item counter of the persistent march
@@ -534,41 +659,6 @@ struct DeviceTemps {
     return e;
   }
 };
-
-float aabb_volume(const float* mn, const float* mx) {
-  float v = 1.0f;
-  for (int a = 0; a < 3; ++a) v *= std::max(mx[a] - mn[a], 1.0e-6f);
-  return v;
-}
-
-// Leaves evaluated exactly at every far-field step instead of being cached:
-// the few whose box dwarfs the box of all remaining leaves (a ground slab).
-std::vector<int> choose_exact_leaves(const ftgpu::SceneImage& im) {
-  const int n = static_cast<int>(im.leaves.size());
-  std::vector<int> order(n);
-  for (int i = 0; i < n; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return aabb_volume(im.leaves[a].bmin, im.leaves[a].bmax) > aabb_volume(im.leaves[b].bmin, im.leaves[b].bmax);
-  });
-  std::vector<int> exact;
-  std::vector<char> is_exact(n, 0);
-  for (int k = 0; k < n - 1 && static_cast<int>(exact.size()) < kMaxExactLeaves; ++k) {
-    int i = order[k];
-    float mn[3] = {kInf, kInf, kInf}, mx[3] = {-kInf, -kInf, -kInf};
-    for (int j = 0; j < n; ++j) {
-      if (j == i || is_exact[j]) continue;
-      for (int a = 0; a < 3; ++a) {
-        mn[a] = std::min(mn[a], im.leaves[j].bmin[a]);
-        mx[a] = std::max(mx[a], im.leaves[j].bmax[a]);
-      }
-    }
-    if (aabb_volume(im.leaves[i].bmin, im.leaves[i].bmax) <= 8.0f * aabb_volume(mn, mx)) break;
-    exact.push_back(i);
-    is_exact[i] = 1;
-  }
-  return exact;
-}
-
 
 // Device tables of one kernel's share of a batch (depth or trace items).
 struct BatchPart {

@@ -321,22 +321,40 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(
     } else {
       q = pos;
     }
-    if (phase == kWfFinal) {
-      WHit h{};
-      Info fin = scene_distance_leaf(S, pos, &h.leaf, cx);
+    // One evaluation site for every phase.  The short scene forms name the
+    // nearest primitive, whose record holds its leaf; the general walk's final
+    // lookup is its own (a lane in its final phase would keep the others
+    // waiting through a second evaluation).
+    const bool final = phase == kWfFinal, general = S.fast.kind == kFastNone;
+    WHit h{};
+    Info info{0.0f, ftd::kNoRef};
+    if (!(final && general)) {
+      const unsigned long long boxes = kStats ? cx.c.boxes : 0ull;
+      info = scene_distance_inl(S, q, cx);
+      if (kStats && final) cx.c.boxes = boxes;  // (the lookup of a hit's leaf is not counted as a cull)
+    }
+    if (final) {
+      if (info.ref < 0) {
+        h.leaf = static_cast<int32_t>(__float_as_uint(__ldg(S.cprims + 3 * static_cast<size_t>(~info.ref) + 2).w) &
+                                      ~ftd::kRareFlag);
+      } else {
+        const unsigned long long evals = kStats ? cx.c.evals : 0ull;
+        info = scene_distance_leaf(S, pos, &h.leaf, cx);
+        if (kStats && !general) cx.c.evals = evals;
+      }
       F3 nn = f3(nx, ny, nz);
       F3 nr = ftd::len3(nn) > 1.0e-8f ? ftd::normalize3(nn) : f3(0.0f, 1.0f, 0.0f);
       h.t = hi;
       h.pos[0] = pos.x; h.pos[1] = pos.y; h.pos[2] = pos.z;
       h.normal[0] = nr.x; h.normal[1] = nr.y; h.normal[2] = nr.z;
-      const uint2 ids = surface_ids(S, fin.ref);
+      const uint2 ids = surface_ids(S, info.ref);
       h.mat = ids.y;
       h.obj = ids.x;
       hits[job] = h;
       live = false;
       continue;
     }
-    const float dq = scene_distance_inl(S, q, cx).d;
+    const float dq = info.d;
     if (phase == kWfMarch) {
       if (fabsf(dq) < eps) {
         lo = prev;
@@ -371,26 +389,40 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(
 }
 
 // A step of shadow_visibility (R:4706-4733): the leaf-box lower bound when it
-// exceeds max(8 eps, 0.02), else the exact distance.  The short scene form
-// computes its box bounds once for both.
+// exceeds max(8 eps, 0.02), else the exact distance.  The short scene forms
+// compute their box bounds once for both; a hard union's bound is 0 inside the
+// box of any primitive that is evaluated at every point (a ground).
 template <bool kStats>
 __device__ __forceinline__ float shadow_step_h(const DevScene& S, F3 p, float eps, Ctx<kStats>& cx) {
   const DevFast& F = S.fast;
   const float least = fmaxf(eps * 8.0f, 0.02f);
-  if (F.kind == kFastTree) {
-    const float t2 = ftd::aabb_lb2(p, F.tmin, F.tmax);
-    const bool alone = F.prim == kNoPrim;
-    const float p2 = alone ? kInf : ftd::aabb_lb2(p, F.pmin, F.pmax);
-    cx.box(alone ? 1 : 3);
-    const float lower = sqrtf(fminf(t2, p2));
-    if (lower > least) return lower;
-    cx.eval();
-    return fabsf(alone ? eval_urtree(S, F.tree, p, kInf, cx).d : tree_and_prim(S, p, t2, p2, cx).d);
+  float l2 = kInf, r2 = kInf, lower;
+  if (F.kind == kFastTree || F.kind == kFastPair) {
+    if (F.entry[0] != kNoPrim) l2 = ftd::aabb_lb2(p, F.bmin[0], F.bmax[0]);
+    r2 = ftd::aabb_lb2(p, F.bmin[1], F.bmax[1]);
+    cx.box(F.entry[0] == kNoPrim ? 1 : 3);
+    lower = sqrtf(fminf(l2, r2));
+  } else {
+    bool known = false;
+    if (F.kind == kFastUnion) {
+      for (int i = 0; i < F.n_always; ++i) {
+        const DevNode& n = S.nodes[__float_as_int(__ldg(S.cprims + 3 * i + 2).z)];
+        cx.box();
+        l2 = fminf(l2, ftd::aabb_lb2(p, n.bmin, n.bmax));
+      }
+      known = F.all || l2 == 0.0f;
+    }
+    lower = known ? sqrtf(l2) : fabsf(scene_lower_bound(S, p, cx));
   }
-  const float lower = fabsf(scene_lower_bound(S, p, cx));
   if (lower > least) return lower;
   cx.eval();
-  return fabsf(scene_distance_general(S, p, cx).d);
+  Info h;
+  if (F.kind == kFastUnion) h = union_distance(S, p, cx);
+  else if (F.kind == kFastNone) h = scene_distance_general(S, p, cx);
+  else if (F.kind == kFastPair) h = pair_distance(S, p, l2, r2, cx);
+  else if (F.entry[0] == kNoPrim) h = eval_urtree(S, F.tree, p, kInf, cx);
+  else h = tree_and_prim(S, p, r2, l2, cx);
+  return fabsf(h.d);
 }
 
 // shadow_visibility (R:4706-4733) of every queued shadow job, one step per

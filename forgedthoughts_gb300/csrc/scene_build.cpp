@@ -125,6 +125,11 @@ class Builder {
         img_->cprims.push_back(compact_prim(lv[1 - k].node, lv[1 - k]));
       }
     }
+    img_->fast_union = std::all_of(lv.begin(), lv.end(), [&](const HostLeaf& l) {
+      return l.kind == kLeafPrim && sane_prim(img_->nodes[l.node]);
+    });
+    if (img_->fast_union)
+      for (const HostLeaf& l : lv) img_->cprims.push_back(compact_prim(l.node, l));
     return true;
   }
 
@@ -960,6 +965,51 @@ bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* 
   *out = SceneImage{};
   Builder b(desc, out, error, lists);
   return b.run();
+}
+
+void build_far_tree(const SceneImage& img, const std::vector<CompactPrim>& prims, int32_t first, int32_t n,
+                    std::vector<FarNode>* nodes, std::vector<uint32_t>* entries) {
+  std::vector<int32_t> idx(n);
+  std::iota(idx.begin(), idx.end(), first);
+  auto box = [&](int32_t i) -> const HostNode& { return img.nodes[prims[i].node]; };
+  // median splits of the box centres along their widest axis
+  std::function<void(size_t, size_t)> build = [&](size_t lo, size_t hi) {
+    const size_t self = nodes->size();
+    FarNode node;
+    node.prims = -1;
+    float cmn[3], cmx[3];
+    for (int a = 0; a < 3; ++a) {
+      node.bmin[a] = cmn[a] = std::numeric_limits<float>::infinity();
+      node.bmax[a] = cmx[a] = -std::numeric_limits<float>::infinity();
+    }
+    for (size_t k = lo; k < hi; ++k)
+      for (int a = 0; a < 3; ++a) {
+        const HostNode& b = box(idx[k]);
+        node.bmin[a] = std::min(node.bmin[a], b.bmin[a]);
+        node.bmax[a] = std::max(node.bmax[a], b.bmax[a]);
+        const float c = (b.bmin[a] + b.bmax[a]) * 0.5f;
+        cmn[a] = std::min(cmn[a], c);
+        cmx[a] = std::max(cmx[a], c);
+      }
+    nodes->push_back(node);
+    if (hi - lo <= static_cast<size_t>(kFarLeaf)) {
+      (*nodes)[self].prims = static_cast<int32_t>(entries->size() << 3 | (hi - lo));
+      for (size_t k = lo; k < hi; ++k)
+        entries->push_back(static_cast<uint32_t>(idx[k]) | (prims[idx[k]].leaf & 0x80000000u));
+    } else {
+      int axis = 0;
+      for (int a = 1; a < 3; ++a)
+        if (cmx[a] - cmn[a] > cmx[axis] - cmn[axis]) axis = a;
+      const size_t mid = (lo + hi) / 2;
+      std::nth_element(idx.begin() + lo, idx.begin() + mid, idx.begin() + hi, [&](int32_t x, int32_t y) {
+        return box(x).bmin[axis] + box(x).bmax[axis] < box(y).bmin[axis] + box(y).bmax[axis];
+      });
+      build(lo, mid);
+      build(mid, hi);
+    }
+    (*nodes)[self].skip = static_cast<int32_t>(nodes->size());
+  };
+  if (n > 0) build(0, static_cast<size_t>(n));
 }
 
 // parse_camera (R:6263-6286) + PinholeCamera::generate_ray basis

@@ -106,8 +106,11 @@ struct SceneImage {
   // A scene of one union_round tree, alone or beside one primitive: their
   // leaves, -1 for other scenes (and no primitive).
   int32_t fast_tree = -1, fast_prim = -1;
-  // compact records of the union_round trees' primitives, indexed as ur_prims,
-  // then that of fast_prim; root paths of the trees' primitives
+  // All leaves are primitives whose boxes bound their distances.
+  bool fast_union = false;
+  // compact records: of the union_round trees' primitives, indexed as ur_prims,
+  // then that of fast_prim; of every leaf, in leaf order, of a fast_union scene.
+  // Root paths of the trees' primitives.
   std::vector<CompactPrim> cprims;
   std::vector<UrPath> ur_paths;
   // per ur_inner node: 1 when its primitives use more than one material model
@@ -134,6 +137,22 @@ struct SceneImage {
 // (ft_scene_build_info reports them); without, only the grids' geometry: a
 // scene on a device builds its own lists there.
 bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error, bool lists);
+
+// Tree over compact primitives for points outside their candidate grids, in
+// depth-first order: a walk goes to the next node, or past a subtree whose box
+// is out of reach, and needs no stack.
+struct FarNode {
+  float bmin[3];
+  int32_t skip;  // the node after the subtree
+  float bmax[3];
+  int32_t prims;  // -1: inner; else (first far entry << 3) | entries
+};
+static_assert(sizeof(FarNode) == 32, "FarNode layout");
+constexpr int kFarLeaf = 4;
+// Appends the tree of the compact primitives [first, first + n) and its
+// entries (compact index | rare flag).
+void build_far_tree(const SceneImage& img, const std::vector<CompactPrim>& prims, int32_t first, int32_t n,
+                    std::vector<FarNode>* nodes, std::vector<uint32_t>* entries);
 
 // Camera basis (R:6263-6286, render_api.rs:132-144) in f32.
 struct CameraBasis {
