@@ -53,39 +53,14 @@ struct DevBricks {
 // R:743-786, with those leaves left out): the field the cache samples.
 template <bool kStats>
 __device__ Info scene_distance_skip(const DevScene& S, F3 p, const DevBricks& B, Ctx<kStats>& cx) {
-  float best = kInf;
   Info cur{kInf, ftd::kNoRef};
-  int stack[64];
-  float stack_lb[64];
-  int sp = 0;
-  stack[sp] = S.bvh_root;
-  stack_lb[sp] = node_lb(p, S.bvh[S.bvh_root].bmin, S.bvh[S.bvh_root].bmax);
-  ++sp;
-  for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
-    --sp;
-    int ni = stack[sp];
-    if (stack_lb[sp] > best) continue;
-    const DevBvhNode& n = S.bvh[ni];
-    if (n.leaf >= 0) {
-      bool skip = false;
-      for (int i = 0; i < B.n_exact; ++i) skip |= (B.exact_leaf[i] == n.leaf);
-      if (skip) continue;
-      Info in = eval_leaf(S, S.leaves[n.leaf], p, best, cx);
-      if (in.d < best) {
-        best = in.d;
-        cur = in;
-      }
-      continue;
-    }
-    float ll = node_lb(p, S.bvh[n.lhs].bmin, S.bvh[n.lhs].bmax), rl = node_lb(p, S.bvh[n.rhs].bmin, S.bvh[n.rhs].bmax);
-    if (sp + 2 > 64) break;
-    if (ll <= rl) {
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-    } else {
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
-    }
+  LeafWalk<kStats> walk(S, p, cx);
+  for (int leaf; (leaf = walk.next(S, cur.d, cx)) >= 0;) {
+    bool skip = false;
+    for (int i = 0; i < B.n_exact; ++i) skip |= (B.exact_leaf[i] == leaf);
+    if (skip) continue;
+    const Info in = eval_leaf(S, S.leaves[leaf], p, cur.d, cx);
+    if (in.d < cur.d) cur = in;
   }
   return cur;
 }

@@ -86,6 +86,7 @@ struct DevScene {
   const DevNode* __restrict__ nodes;
   const DevLeaf* __restrict__ leaves;
   const DevBvhNode* __restrict__ bvh;
+  const float4* __restrict__ bvh_pairs;  // per inner node of bvh: { lmin, lhs } { lmax, - } { rmin, rhs } { rmax, - }
   const uint32_t* __restrict__ gops;
   const DevUrTree* __restrict__ urtrees;
   const DevUrBvh* __restrict__ ur_bvh;
@@ -109,6 +110,7 @@ struct DevScene {
   int32_t n_obj_node;
   int32_t n_materials, n_lights, env_program;
   int32_t bvh_root;
+  int32_t bvh_ref;  // the root as a pair reference: an index into bvh_pairs, or ~leaf
   float smin[3], smax[3];
 };
 
@@ -607,6 +609,85 @@ __device__ __forceinline__ Info eval_urtree(const DevScene& S, const DevUrTree& 
   return ur_value(S, t, n, near_idx, near_dist, p, cx);
 }
 
+// A leaf [distance_post] [domain] primitive, the common form of a hooked
+// object, in registers: the steps of its postfix program (eval_generic keeps
+// its operands in local memory).
+template <bool kStats>
+__device__ __noinline__ Info eval_hooked(const DevScene& S, int node, F3 p, Ctx<kStats>& cx) {
+  const DevNode* n = &S.nodes[node];
+  const DevNode* post = nullptr;
+  F3 pp = p;
+  if (n->kind == FT_NODE_DISTANCE_POST) {
+    post = n;
+    pp = ftd::to_local(p, *n);
+    node = n->a;
+    n = &S.nodes[node];
+  }
+  F3 q = pp;
+  if (n->kind == FT_NODE_DOMAIN) {
+    F3 local = ftd::to_local(pp, *n);
+    q = scene_program(S, n->program, &local, cx.hooks());
+    node = n->a;
+    n = &S.nodes[node];
+  }
+  cx.prim();
+  float d = ftd::prim_distance(*n, q);
+  if (post) {
+    F3 args[2] = {f3(d, d, d), pp};
+    d = scene_program(S, post->program, args, cx.hooks()).x;
+  }
+  return Info{d, node};
+}
+
+// The leaves of the leaf BVH in the order of bvh_distance_info (R:743-786):
+// nearest child first, a node left out when its box bound exceeds the best
+// distance at that time.  next() descends to the next leaf and returns, so
+// the lanes of a warp reach their leaves' evaluations together instead of
+// half of them waiting on box tests.  A node's two child boxes are four
+// 16-byte loads; the nearer child stays in registers.
+template <bool kStats>
+struct LeafWalk {
+  static constexpr int kStack = 48;  // (the median-split build is about log2(leaves) deep)
+  F3 p;
+  int ref, sp = 0;
+  float lb;
+  bool have = true;
+  int stack[kStack];
+  float bound[kStack];
+  __device__ __forceinline__ LeafWalk(const DevScene& S, F3 q, Ctx<kStats>& cx) : p(q), ref(S.bvh_ref) {
+    lb = node_lb(q, S.smin, S.smax);
+    cx.box();
+  }
+  // Next leaf whose bound is not above `best`, -1 at the end; its bound is lb.
+  __device__ __forceinline__ int next(const DevScene& S, float best, Ctx<kStats>& cx) {
+    for (int walk = 0; walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk visits each node once
+      if (!have) {
+        if (sp == 0) return -1;
+        --sp;
+        ref = stack[sp];
+        lb = bound[sp];
+      }
+      have = false;
+      if (lb > best) continue;
+      if (ref < 0) return ~ref;
+      const float4* w = S.bvh_pairs + 4 * static_cast<size_t>(ref);
+      const float4 a = __ldg(w), b = __ldg(w + 1), c = __ldg(w + 2), e = __ldg(w + 3);
+      const float lmn[3] = {a.x, a.y, a.z}, lmx[3] = {b.x, b.y, b.z}, rmn[3] = {c.x, c.y, c.z}, rmx[3] = {e.x, e.y, e.z};
+      const float ll = node_lb(p, lmn, lmx), rl = node_lb(p, rmn, rmx);
+      cx.box(2);
+      if (sp == kStack) return -1;  // deeper than the build makes it
+      const bool lfirst = ll <= rl;
+      stack[sp] = __float_as_int(lfirst ? c.w : a.w);
+      bound[sp] = lfirst ? rl : ll;
+      ++sp;
+      ref = __float_as_int(lfirst ? a.w : c.w);
+      lb = lfirst ? ll : rl;
+      have = true;
+    }
+    return -1;
+  }
+};
+
 template <bool kStats>
 __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, F3 p, float cutoff, Ctx<kStats>& cx) {
   if (lf.kind == ftgpu::kLeafPrim) {
@@ -614,6 +695,7 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, 
     cx.prim();
     return Info{ftd::prim_distance(n, p), lf.node};
   }
+  if (lf.kind == ftgpu::kLeafHooked) return eval_hooked(S, lf.node, p, cx);
   if (lf.kind == ftgpu::kLeafUrTree) return eval_urtree(S, S.urtrees[lf.first], p, cutoff, cx);
   if (S.nodes[lf.node].kind == FT_NODE_CUSTOM) {
     // accel_leaf_distance_info (R:635-657): a Custom leaf farther from its box
@@ -635,41 +717,11 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, 
 // closer.
 template <bool kStats>
 __device__ __noinline__ Info scene_distance_bvh(const DevScene& S, F3 p, Ctx<kStats>& cx) {
-  float best = kInf;
   Info cur{kInf, ftd::kNoRef};
-  int stack[64];
-  float stack_lb[64];
-  int sp = 0;
-  stack[sp] = S.bvh_root;
-  stack_lb[sp] = node_lb(p, S.bvh[S.bvh_root].bmin, S.bvh[S.bvh_root].bmax);
-  ++sp;
-  cx.box();
-  for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
-    --sp;
-    int ni = stack[sp];
-    if (stack_lb[sp] > best) continue;
-    const DevBvhNode& n = S.bvh[ni];
-    if (n.leaf >= 0) {
-      Info in = eval_leaf(S, S.leaves[n.leaf], p, best, cx);
-      if (in.d < best) {
-        best = in.d;
-        cur = in;
-      }
-      continue;
-    }
-    const DevBvhNode& L = S.bvh[n.lhs];
-    const DevBvhNode& R = S.bvh[n.rhs];
-    float ll = node_lb(p, L.bmin, L.bmax), rl = node_lb(p, R.bmin, R.bmax);
-    cx.box();
-    cx.box();
-    if (sp + 2 > 64) break;  // depth is bounded by the median-split build
-    if (ll <= rl) {
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-    } else {
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
-    }
+  LeafWalk<kStats> walk(S, p, cx);
+  for (int leaf; (leaf = walk.next(S, cur.d, cx)) >= 0;) {
+    const Info in = eval_leaf(S, S.leaves[leaf], p, cur.d, cx);
+    if (in.d < cur.d) cur = in;
   }
   return cur;
 }
@@ -835,39 +887,19 @@ __device__ __forceinline__ float scene_d(const DevScene& S, F3 p, Ctx<kStats>& c
 template <bool kStats>
 __device__ __noinline__ Info scene_distance_leaf(const DevScene& S, F3 p, int* leaf, Ctx<kStats>& cx) {
   cx.eval();
-  float best = kInf;
   Info cur{kInf, ftd::kNoRef};
-  *leaf = 0;
-  int stack[64];
-  float stack_lb[64];
-  int sp = 0;
-  stack[sp] = S.bvh_root;
-  stack_lb[sp] = node_lb(p, S.bvh[S.bvh_root].bmin, S.bvh[S.bvh_root].bmax);
-  ++sp;
-  for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
-    --sp;
-    int ni = stack[sp];
-    if (stack_lb[sp] > best) continue;
-    const DevBvhNode& n = S.bvh[ni];
-    if (n.leaf >= 0) {
-      Info in = eval_leaf(S, S.leaves[n.leaf], p, best, cx);
-      if (in.d < best) {
-        best = in.d;
-        cur = in;
-        *leaf = n.leaf;
-      }
-      continue;
-    }
-    float ll = node_lb(p, S.bvh[n.lhs].bmin, S.bvh[n.lhs].bmax), rl = node_lb(p, S.bvh[n.rhs].bmin, S.bvh[n.rhs].bmax);
-    if (sp + 2 > 64) break;
-    if (ll <= rl) {
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-    } else {
-      stack[sp] = n.lhs; stack_lb[sp] = ll; ++sp;
-      stack[sp] = n.rhs; stack_lb[sp] = rl; ++sp;
+  int nearest = 0;
+  const unsigned long long boxes = cx.c.boxes;
+  LeafWalk<kStats> walk(S, p, cx);
+  for (int li; (li = walk.next(S, cur.d, cx)) >= 0;) {
+    const Info in = eval_leaf(S, S.leaves[li], p, cur.d, cx);
+    if (in.d < cur.d) {
+      cur = in;
+      nearest = li;
     }
   }
+  cx.c.boxes = boxes;  // (not counted as culls)
+  *leaf = nearest;
   return cur;
 }
 

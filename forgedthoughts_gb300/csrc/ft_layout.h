@@ -11,7 +11,8 @@ namespace ftgpu {
 enum LeafKind : int32_t {
   kLeafPrim = 0,     // a single primitive node: inline evaluation
   kLeafGeneric = 1,  // postfix program over the leaf's node tree
-  kLeafUrTree = 2    // union_round tree of primitives with one radius
+  kLeafUrTree = 2,   // union_round tree of primitives with one radius
+  kLeafHooked = 3    // (device only) generic leaf of the form [distance_post] [domain] primitive
 };
 
 // Generic-program opcodes (top 5 bits of a uint32 op word, node index below).

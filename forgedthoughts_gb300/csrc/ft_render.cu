@@ -376,19 +376,46 @@ ft_status upload_scene(ft_scene* sc) {
       }
     }
   };
+  // Leaf BVH: each inner node's two child boxes and references
+  std::vector<float4> pairs;
+  std::vector<int32_t> pair_of(im.bvh.size(), -1);
+  int32_t n_pairs = 0;
+  for (size_t k = 0; k < im.bvh.size(); ++k)
+    if (im.bvh[k].leaf < 0) pair_of[k] = n_pairs++;
+  auto bvh_ref = [&](int32_t k) { return im.bvh[k].leaf >= 0 ? ~im.bvh[k].leaf : pair_of[k]; };
+  for (const ftgpu::HostBvhNode& n : im.bvh) {
+    if (n.leaf >= 0) continue;
+    for (int32_t c : {n.lhs, n.rhs}) {
+      const ftgpu::HostBvhNode& b = im.bvh[c];
+      float ref;
+      const int32_t r = bvh_ref(c);
+      std::memcpy(&ref, &r, sizeof(ref));
+      pairs.push_back(make_float4(b.bmin[0], b.bmin[1], b.bmin[2], ref));
+      pairs.push_back(make_float4(b.bmax[0], b.bmax[1], b.bmax[2], 0.0f));
+    }
+  }
+  // Leaves with their device kinds: [distance_post] [domain] primitive
+  std::vector<ftgpu::HostLeaf> leaves = im.leaves;
+  for (ftgpu::HostLeaf& l : leaves) {
+    if (l.kind != ftgpu::kLeafGeneric) continue;
+    int32_t k = l.node;
+    if (im.nodes[k].kind == FT_NODE_DISTANCE_POST) k = im.nodes[k].a;
+    if (im.nodes[k].kind == FT_NODE_DOMAIN) k = im.nodes[k].a;
+    if (k != l.node && im.nodes[k].kind <= FT_NODE_EXTRUDE_POLYGON) l.kind = ftgpu::kLeafHooked;
+  }
   std::vector<Part> parts;
   auto part = [&](const void* src, size_t bytes) {
     parts.push_back(Part{src, bytes, 0});
     return parts.size() - 1;
   };
   auto vec = [&](const auto& v) { return part(v.data(), v.size() * sizeof(v[0])); };
-  const size_t p_nodes = vec(im.nodes), p_leaves = vec(im.leaves), p_bvh = vec(im.bvh), p_gops = vec(im.gops),
+  const size_t p_nodes = vec(im.nodes), p_leaves = vec(leaves), p_bvh = vec(im.bvh), p_gops = vec(im.gops),
                p_trees = vec(trees), p_ur_bvh = vec(im.ur_bvh), p_ur_bvh_prims = vec(im.ur_bvh_prims),
                p_ur_prims = vec(im.ur_prims), p_ur_inner = vec(im.ur_inner), p_programs = vec(im.programs),
                p_instrs = vec(im.instrs), p_cprims = vec(cprims), p_paths = vec(im.ur_paths),
                p_materials = vec(im.materials), p_lights = vec(im.lights), p_op_begin = vec(im.node_op_begin),
                p_op_end = vec(im.node_op_end), p_blend = vec(im.ur_inner_blend), p_obj = vec(im.obj_node),
-               p_far = vec(far_nodes), p_far_entries = vec(far_entries);
+               p_far = vec(far_nodes), p_far_entries = vec(far_entries), p_pairs = vec(pairs);
   size_t total = 0;
   for (Part& p : parts) {
     p.off = total;
@@ -425,6 +452,8 @@ ft_status upload_scene(ft_scene* sc) {
   at(p_blend, d.ur_inner_blend);
   at(p_obj, d.obj_node);
   at(p_far, d.far_nodes);
+  at(p_pairs, d.bvh_pairs);
+  d.bvh_ref = bvh_ref(im.bvh_root);
   at(p_far_entries, d.far_entries);
   d.n_obj_node = static_cast<int32_t>(im.obj_node.size());
   d.n_materials = static_cast<int32_t>(im.materials.size());

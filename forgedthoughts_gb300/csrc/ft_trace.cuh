@@ -868,32 +868,8 @@ __device__ float scene_lower_bound(const DevScene& S, F3 p, Ctx<kStats>& cx) {
     }
   }
   float best = kInf;
-  cx.box();
-  int stack[64];
-  float slb[64];
-  int sp = 0;
-  stack[0] = S.bvh_root;
-  slb[0] = node_lb(p, S.bvh[S.bvh_root].bmin, S.bvh[S.bvh_root].bmax);
-  sp = 1;
-  for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
-    --sp;
-    if (slb[sp] > best) continue;
-    const DevBvhNode& n = S.bvh[stack[sp]];
-    if (n.leaf >= 0) {
-      best = fminf(best, slb[sp]);
-      continue;
-    }
-    if (sp + 2 > 64) break;
-    float ll = node_lb(p, S.bvh[n.lhs].bmin, S.bvh[n.lhs].bmax), rl = node_lb(p, S.bvh[n.rhs].bmin, S.bvh[n.rhs].bmax);
-    cx.box(2);
-    if (ll <= rl) {
-      stack[sp] = n.rhs; slb[sp] = rl; ++sp;
-      stack[sp] = n.lhs; slb[sp] = ll; ++sp;
-    } else {
-      stack[sp] = n.lhs; slb[sp] = ll; ++sp;
-      stack[sp] = n.rhs; slb[sp] = rl; ++sp;
-    }
-  }
+  LeafWalk<kStats> walk(S, p, cx);
+  while (walk.next(S, best, cx) >= 0) best = fminf(best, walk.lb);
   return best;
 }
 
