@@ -688,6 +688,14 @@ struct LeafWalk {
   }
 };
 
+// The general leaf walk's tree evaluation, out of line (the short scene form
+// inlines its own).
+template <bool kStats>
+__device__ __noinline__ Info eval_urtree_leaf(const DevScene& S, const DevUrTree& t, F3 p, float cutoff,
+                                              Ctx<kStats>& cx) {
+  return eval_urtree(S, t, p, cutoff, cx);
+}
+
 template <bool kStats>
 __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, F3 p, float cutoff, Ctx<kStats>& cx) {
   if (lf.kind == ftgpu::kLeafPrim) {
@@ -696,7 +704,7 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, const DevLeaf& lf, 
     return Info{ftd::prim_distance(n, p), lf.node};
   }
   if (lf.kind == ftgpu::kLeafHooked) return eval_hooked(S, lf.node, p, cx);
-  if (lf.kind == ftgpu::kLeafUrTree) return eval_urtree(S, S.urtrees[lf.first], p, cutoff, cx);
+  if (lf.kind == ftgpu::kLeafUrTree) return eval_urtree_leaf(S, S.urtrees[lf.first], p, cutoff, cx);
   if (S.nodes[lf.node].kind == FT_NODE_CUSTOM) {
     // accel_leaf_distance_info (R:635-657): a Custom leaf farther from its box
     // than a tenth of the box diagonal (clamped to [0.05, 0.5]) is that box

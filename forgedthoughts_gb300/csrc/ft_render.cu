@@ -111,6 +111,7 @@ struct ft_scene {
   size_t cap_items = 0, cap_pixels = 0;
   unsigned long long* d_stats = nullptr;
   int persistent_blocks = 1;
+  int sms = 1;
   // FP16 brick cache (ft_scene_build_bricks)
   bool has_bricks = false;
   DevBricks bricks{};
@@ -531,6 +532,7 @@ ft_status upload_scene(ft_scene* sc) {
   FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, false, false>, 128, 0),
               "occupancy");
   sc->persistent_blocks = std::max(1, sms * std::max(per_sm, 1));
+  sc->sms = std::max(1, sms);
   FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, true, false>, 128, 0),
               "occupancy");
   sc->persistent_blocks_bricks = std::max(1, sms * std::max(per_sm, 1));
@@ -2002,6 +2004,15 @@ std::vector<RayParams> view_params(const ft_scene* sc, const ft_view* views, uin
   return out;
 }
 
+// Rays of one pass of the adjoint (24 bytes of records each).
+constexpr uint64_t kAdjointChunk = uint64_t(1) << 22;
+
+// Blocks of a views pass over n rays: five per SM, its resident blocks.
+unsigned view_blocks(const ft_scene* sc, uint64_t n) {
+  const uint64_t resident = static_cast<uint64_t>(sc->sms) * 5;
+  return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n + 127) / 128, resident)));
+}
+
 ft_status check_views(const ft_scene* sc, const ft_view* views, uint32_t n, const ft_render_options* o, float tau) {
   if (!sc || !views || n == 0) return ftcommon::fail(FT_ERR_INVALID_ARGUMENT, "scene and views must be non-null");
   if (ft_status s = check_options(o, 1)) return s;
@@ -2033,16 +2044,23 @@ ft_status ft_render_views(ft_scene* sc, const ft_view* views, uint32_t n_views, 
     if (mask_out) FT_CUDA_TRY(tmp.alloc(&m, total_px), "cudaMalloc(mask)");
     if (sil_out) FT_CUDA_TRY(tmp.alloc(&sil, total_px), "cudaMalloc(silhouette)");
   }
-  uint64_t threads = items * n_views;
-  views_forward_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(sc->dev, d_views, n_views, items,
-                                                                                     tau, t, m, sil);
-  FT_CUDA_TRY(cudaGetLastError(), "views_forward_kernel launch");
+  unsigned long long* d_counters = nullptr;
+  FT_CUDA_TRY(tmp.alloc(&d_counters, kViewCounters), "cudaMalloc(counters)");
+  FT_CUDA_TRY(cudaMemsetAsync(d_counters, 0, kViewCounters * sizeof(unsigned long long), st), "memset");
+  const uint64_t n_work = items * n_views;
+  views_march_persistent<false><<<view_blocks(sc, n_work), 128, 0, st>>>(sc->dev, d_views, items, 0, n_work, tau, t, m,
+                                                                         sil, nullptr, nullptr, nullptr, d_counters);
+  FT_CUDA_TRY(cudaGetLastError(), "views_march_persistent launch");
+  unsigned long long march_flags = 0;
+  FT_CUDA_TRY(cudaMemcpyAsync(&march_flags, d_counters + 1, sizeof(march_flags), cudaMemcpyDeviceToHost, st),
+              "march flags");
   if (!dev_ptrs) {
     if (t_out) FT_CUDA_TRY(cudaMemcpyAsync(t_out, t, total_px * sizeof(float), cudaMemcpyDeviceToHost, st), "copy");
     if (mask_out) FT_CUDA_TRY(cudaMemcpyAsync(mask_out, m, total_px, cudaMemcpyDeviceToHost, st), "copy");
     if (sil_out) FT_CUDA_TRY(cudaMemcpyAsync(sil_out, sil, total_px * sizeof(float), cudaMemcpyDeviceToHost, st), "copy");
   }
   FT_CUDA_TRY(cudaStreamSynchronize(st), "views");
+  if (ft_status s = march_check(march_flags)) return s;
   ftcommon::clear_last_error();
   return FT_OK;
   FT_API_END
@@ -2122,13 +2140,30 @@ ft_status ft_render_backward(ft_scene* sc, const ft_view* views, uint32_t n_view
   DiffTables T{d_slot, d_tree, n_params};
   const size_t smem = static_cast<size_t>(n_params) * sizeof(double);
   const int shared_acc = (n_params > 0 && smem <= 48 * 1024) ? 1 : 0;
-  int sms = 0;
-  FT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sc->device), "sm count");
-  uint64_t want = (items * n_views + 127) / 128;
-  unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(want, static_cast<uint64_t>(sms) * 8)));
-  views_backward_kernel<<<grid, 128, shared_acc ? smem : 0, st>>>(sc->dev, d_views, n_views, items, tau, T, a, b,
-                                                                  d_grad, shared_acc, d_bad);
-  FT_CUDA_TRY(cudaGetLastError(), "views_backward_kernel launch");
+  // In chunks of rays, which bounds the records' memory: march them again,
+  // then take the gradient of those that count.
+  const uint64_t total = items * n_views, chunk = std::min<uint64_t>(total, kAdjointChunk);
+  AdjointRay* d_rays = nullptr;
+  unsigned long long* d_counters = nullptr;
+  FT_CUDA_TRY(tmp.alloc(&d_rays, chunk), "cudaMalloc(adjoint rays)");
+  FT_CUDA_TRY(tmp.alloc(&d_counters, kViewCounters), "cudaMalloc(counters)");
+  FT_CUDA_TRY(cudaMemsetAsync(d_counters, 0, kViewCounters * sizeof(unsigned long long), st), "memset");
+  for (uint64_t first = 0; first < total; first += chunk) {
+    const uint64_t n = std::min(chunk, total - first);
+    // (the self-check flags, counter 1, collect over the chunks)
+    FT_CUDA_TRY(cudaMemsetAsync(d_counters, 0, sizeof(unsigned long long), st), "memset");
+    FT_CUDA_TRY(cudaMemsetAsync(d_counters + 2, 0, 2 * sizeof(unsigned long long), st), "memset");
+    const unsigned grid = view_blocks(sc, n);
+    views_march_persistent<true><<<grid, 128, 0, st>>>(sc->dev, d_views, items, first, n, tau, nullptr, nullptr,
+                                                       nullptr, a, b, d_rays, d_counters);
+    FT_CUDA_TRY(cudaGetLastError(), "views_march_persistent launch");
+    views_adjoint_kernel<<<grid, 128, shared_acc ? smem : 0, st>>>(sc->dev, d_views, items, n, tau, T, d_rays,
+                                                                   d_counters, d_grad, shared_acc, d_bad);
+    FT_CUDA_TRY(cudaGetLastError(), "views_adjoint_kernel launch");
+  }
+  unsigned long long march_flags = 0;
+  FT_CUDA_TRY(cudaMemcpyAsync(&march_flags, d_counters + 1, sizeof(march_flags), cudaMemcpyDeviceToHost, st),
+              "march flags");
   int bad = 0;
   FT_CUDA_TRY(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st), "copy");
   if (dev_ptrs)
@@ -2136,6 +2171,7 @@ ft_status ft_render_backward(ft_scene* sc, const ft_view* views, uint32_t n_view
   else
     FT_CUDA_TRY(cudaMemcpyAsync(dL_dparams, d_grad, n_params * sizeof(double), cudaMemcpyDeviceToHost, st), "copy");
   FT_CUDA_TRY(cudaStreamSynchronize(st), "backward");
+  if (ft_status s = march_check(march_flags)) return s;
   if (bad) return ftcommon::fail(FT_ERR_UNSUPPORTED, "the hit leaf is not a union_round tree of spheres / boxes "
                                                      "(or has more than 512 primitives): no adjoint");
   ftcommon::clear_last_error();
