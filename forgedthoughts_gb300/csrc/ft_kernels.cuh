@@ -44,6 +44,10 @@ struct alignas(16) DevGrid {
   int32_t dims[3];
   int32_t first;
 };
+// Distance up to which a cell lists every primitive: a little above the blend
+// radius, so that a hit (whose own distance is at most epsilon) finds all the
+// primitives with a weight in its normal and material in its cell's list.
+__host__ __device__ inline float ur_list_reach(float r) { return 1.05f * r + 1.0e-3f; }
 struct DevUrTree {
   float r;
   int32_t n_prims, prim_first, bvh_root, inner_root, depth, fallback_first, fallback_count;

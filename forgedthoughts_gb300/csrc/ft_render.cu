@@ -475,7 +475,7 @@ ft_status upload_scene(ft_scene* sc) {
   for (size_t k = 0; k < im.urtrees.size(); ++k) {
     const ftgpu::HostUrTree& t = im.urtrees[k];
     if (t.dims[0] <= 0) continue;
-    jobs.push_back(grid_job(t.gmin, t.cell, t.dims, t.prim_first, t.n_prims, t.r));
+    jobs.push_back(grid_job(t.gmin, t.cell, t.dims, t.prim_first, t.n_prims, ur_list_reach(t.r)));
     owner.emplace_back(k, false);
     if (t.odims[0] <= 0) continue;
     jobs.push_back(grid_job(t.ogmin, t.ocell, t.odims, t.prim_first, t.n_prims, t.r));

@@ -588,28 +588,50 @@ __device__ __noinline__ void resolve_generic(const DevScene& S, int root, F3 p, 
 }
 
 // ---------------------------------------------------------------- union_round trees
-// Gather the primitives within `reach` of p (exact distances) through the
-// tree's BVH.  Returns false when more than kGather qualify.
-__device__ bool ur_gather(const DevScene& S, const DevUrTree& t, F3 p, float reach, int* pos, float* dist, int* n) {
+// Gather the primitives within `reach` of p (exact distances), in tree order.
+// The first reach (ur_list_reach) is what a candidate cell
+// lists in full; a wider one walks the tree's BVH.  Returns false when more
+// than kGather qualify.
+__device__ __noinline__ bool ur_gather(const DevScene& S, const DevUrTree& t, F3 p, float reach, int* pos, float* dist,
+                                       int* n) {
+  int count = 0;
+  auto add = [&](int ps) {
+    const DevNode& pn = S.nodes[S.ur_prims[t.prim_first + ps]];
+    const float d = ftd::prim_distance(pn, p);
+    if (!(d < reach)) return true;
+    if (count >= kGather) return false;
+    int j = count++;
+    for (; j > 0 && pos[j - 1] > ps; --j) {
+      pos[j] = pos[j - 1];
+      dist[j] = dist[j - 1];
+    }
+    pos[j] = ps;
+    dist[j] = d;
+    return true;
+  };
+  int cell = 0;
+  if (reach <= ur_list_reach(t.r) && grid_cell(t.fine, p, &cell)) {
+    const uint2 range = __ldg(S.cells + cell);
+    for (uint32_t k = range.x, end = range.x + range.y; k < end; ++k) {
+      const uint2 e = __ldg(S.entries + k);
+      if (__uint_as_float(e.x) >= reach) break;
+      if (!add(static_cast<int>(e.y & ~ftd::kRareFlag) - t.prim_first)) return false;
+    }
+    *n = count;
+    return true;
+  }
   int stack[48];
   int sp = 0;
-  *n = 0;
   stack[sp++] = t.bvh_root;
   for (int walk = 0; sp > 0 && walk < ftgpu::kMaxWalk; ++walk) {  // a tree walk pops each node once
     const DevUrBvh& bn = S.ur_bvh[stack[--sp]];
     if (node_lb(p, bn.bmin, bn.bmax) >= reach) continue;
     if (bn.prim_count > 0) {
       for (int k = 0; k < bn.prim_count; ++k) {
-        int ps = S.ur_bvh_prims[bn.prim_begin + k];
+        const int ps = S.ur_bvh_prims[bn.prim_begin + k];
         const DevNode& pn = S.nodes[S.ur_prims[t.prim_first + ps]];
         if (node_lb(p, pn.bmin, pn.bmax) >= reach) continue;
-        float d = ftd::prim_distance(pn, p);
-        if (d < reach) {
-          if (*n >= kGather) return false;
-          pos[*n] = ps;
-          dist[*n] = d;
-          ++*n;
-        }
+        if (!add(ps)) return false;
       }
       continue;
     }
@@ -617,63 +639,56 @@ __device__ bool ur_gather(const DevScene& S, const DevUrTree& t, F3 p, float rea
     stack[sp++] = bn.left;
     stack[sp++] = bn.right;
   }
+  *n = count;
   return true;
 }
 
-// Exact value of the union_round subtree `c` (inner index, or -(pos + 1) for
-// a primitive) at p from the gathered primitives; kInf when it holds none
-// (its true value is then >= reach).  Primitives outside the gather are >= the
-// reach, which keeps every union_round on the fold's path exact.
-__device__ float ur_subtree_value(const DevScene& S, const DevUrTree& t, int c, const int* gpos, const float* gdist,
-                                  int ng) {
-  auto prim_value = [&](int ps) {
-    for (int k = 0; k < ng; ++k)
-      if (gpos[k] == ps) return gdist[k];
-    return kInf;
-  };
-  if (c < 0) return prim_value(-c - 1);
-  auto has = [&](int in) {
-    const DevUrInner& u = S.ur_inner[in];
-    for (int k = 0; k < ng; ++k)
-      if (gpos[k] >= u.lo && gpos[k] < u.hi) return true;
-    return false;
-  };
-  if (!has(c)) return kInf;
-  struct VF {
-    int inner, stage;
-    float v[2];
-  };
-  VF fr[24];
-  int fp = 0;
-  fr[0].inner = c;
-  fr[0].stage = 0;
-  for (int walk = 0; walk < ftgpu::kMaxWalk; ++walk) {  // each inner node is opened once
-    VF& F = fr[fp];
-    if (F.stage < 2) {
-      int ch = S.ur_inner[F.inner].child[F.stage];
-      if (ch < 0) {
-        F.v[F.stage++] = prim_value(-ch - 1);
-        continue;
-      }
-      if (!has(ch)) {
-        F.v[F.stage++] = kInf;
-        continue;
-      }
-      if (fp + 1 >= 24) return kInf;  // deeper than supported; the caller widens and falls back
-      ++F.stage;
-      ++fp;
-      fr[fp].inner = ch;
-      fr[fp].stage = 0;
-      continue;
-    }
-    float v = (F.v[0] == kInf && F.v[1] == kInf)
-                  ? kInf
-                  : ftd::op_union_round(F.v[0], F.v[1], t.r);
-    if (fp == 0) return v;
-    --fp;
-    fr[fp].v[fr[fp].stage - 1] = v;
+// Exact value at p of the union_round subtree at `depth` whose gathered
+// primitives are [i0, i1); kInf when it holds none (its true value is then >=
+// reach).  Primitives outside the gather are >= the reach, which keeps every
+// union_round on the fold's path exact.  Joined along root paths, as
+// ur_fold_many.
+__device__ __forceinline__ float ur_lift_far(float v, int levels, float r) {
+  for (int k = 0; k < levels; ++k) {
+    const float up = ur_lift(v, r);
+    if (up == v) break;
+    v = up;
   }
-  return kInf;  // only a corrupted tree gets here
+  return v;
+}
+__device__ __noinline__ float ur_subtree_many(const DevScene& S, const DevUrTree& t, int depth, const int* gpos,
+                                              const float* gdist, int i0, int i1) {
+  struct Open {
+    float v;
+    int at;
+  };
+  Open open[kGather];
+  int sp = 0;
+  uint4 path = __ldg(S.ur_paths + t.prim_first + gpos[i0]);
+  float cur = 0.0f;
+  for (int i = i0; i < i1; ++i) {
+    cur = gdist[i];
+    int dep = static_cast<int>(path.z), l = depth - 1;
+    if (i + 1 < i1) {
+      const uint4 nxt = __ldg(S.ur_paths + t.prim_first + gpos[i + 1]);
+      l = ur_lca(path, nxt);
+      path = nxt;
+    }
+    while (sp > 0 && open[sp - 1].at > l) {
+      --sp;
+      cur = ftd::op_union_round(open[sp].v, ur_lift_far(cur, dep - open[sp].at - 1, t.r), t.r);
+      dep = open[sp].at;
+    }
+    cur = ur_lift_far(cur, dep - l - 1, t.r);
+    if (i + 1 < i1) open[sp++] = Open{cur, l};
+  }
+  return cur;
+}
+__device__ __forceinline__ float ur_subtree_value(const DevScene& S, const DevUrTree& t, int depth, const int* gpos,
+                                                  const float* gdist, int i0, int i1) {
+  if (i0 == i1) return kInf;
+  if (i1 - i0 > 1) return ur_subtree_many(S, t, depth, gpos, gdist, i0, i1);
+  return ur_lift_far(gdist[i0], static_cast<int>(__ldg(S.ur_paths + t.prim_first + gpos[i0]).z) - depth, t.r);
 }
 
 struct NEntry {
@@ -703,6 +718,7 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
   }
   struct Frame {
     int inner, stage;
+    int i0, im, i1;  // gathered primitives of the left and right child
     float tw;
     bool useL, useR;
   };
@@ -713,13 +729,19 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
   int fp = 0;
   const float r = t.r;
   // Set up a frame: child values, exact weight, which children carry weight.
-  auto open = [&](int fi, int inner) -> bool {
+  auto open = [&](int fi, int inner, int i0, int i1) -> bool {
     Frame& F = fr[fi];
     F.inner = inner;
     F.stage = 0;
     const DevUrInner& u = S.ur_inner[inner];
-    float vL = ur_subtree_value(S, t, u.child[0], gpos, gdist, ng);
-    float vR = ur_subtree_value(S, t, u.child[1], gpos, gdist, ng);
+    const int first_right = u.child[1] < 0 ? -u.child[1] - 1 : S.ur_inner[u.child[1]].lo;
+    int im = i0;
+    while (im < i1 && gpos[im] < first_right) ++im;
+    F.i0 = i0;
+    F.im = im;
+    F.i1 = i1;
+    float vL = ur_subtree_value(S, t, fi + 1, gpos, gdist, i0, im);
+    float vR = ur_subtree_value(S, t, fi + 1, gpos, gdist, im, i1);
     if (vL == kInf && vR == kInf) {
       *need = -1.0f;
       return false;
@@ -736,7 +758,7 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
     F.useR = F.tw != 0.0f;
     return true;
   };
-  if (!open(0, t.inner_root)) return false;
+  if (!open(0, t.inner_root, 0, ng)) return false;
   for (int walk = 0; walk < ftgpu::kMaxWalk; ++walk) {  // each inner node is opened once
     Frame& F = fr[fp];
     bool child_done = false;  // carry holds the result of fr[fp]'s child (stage - 1)
@@ -758,9 +780,10 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
           *need = -1.0f;
           return false;
         }
+        const int i0 = F.stage == 0 ? F.i0 : F.im, i1 = F.stage == 0 ? F.im : F.i1;
         ++F.stage;
         ++fp;
-        if (!open(fp, c)) return false;
+        if (!open(fp, c, i0, i1)) return false;
         continue;
       }
     } else {
@@ -812,13 +835,13 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
 
 __device__ void resolve_urtree(const DevScene& S, const DevUrTree& t, F3 p, const HookCtx& hc, Resolved* out,
                                bool split_root) {
-  float reach = 3.0f * t.r;
+  float reach = t.fine.dims[0] > 0 ? ur_list_reach(t.r) : 3.0f * t.r;
   out->ok = false;
   for (int attempt = 0; attempt < 6; ++attempt) {
     float need = 0.0f;
     if (resolve_urtree_reach(S, t, p, hc, reach, out, &need, split_root)) return;
     if (need < 0.0f) return;  // capacity exceeded
-    reach = fmaxf(1.5f * reach, need * 1.0001f + 1.0e-6f);
+    reach = fmaxf(fmaxf(1.5f * reach, 3.0f * t.r), need * 1.0001f + 1.0e-6f);
   }
 }
 
