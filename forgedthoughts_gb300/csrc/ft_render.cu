@@ -135,6 +135,8 @@ struct ft_scene {
   // job counts (2), shadow count, overflow flag, march and shadow work
   // counters, self-check flags (kWfCounters)
   unsigned long long* wf_counters = nullptr;
+  float* path_buf = nullptr;  // path tracer: pixel states, then the samples of a pass
+  uint64_t path_cap = 0;
   uint32_t last_launches = 0;  // kernels launched by the last ft_render_depth / ft_render_trace
   // Per-kernel CUDA-event timing (ft_scene_profile): an event pair around each
   // launch since the last collection, and the sums per kernel kind.
@@ -939,6 +941,9 @@ ft_status check_tuning(const ft_batch_tuning& t) {
 
 
 
+// Path samples of one pass (12 bytes each).
+constexpr uint64_t kPathSamples = uint64_t(1) << 24;
+
 // Whitted trace of one frame as a wavefront: per bounce level one march, one
 // shade and one shadow kernel over queues (ft_wavefront.cuh).  Radiance per
 // sample lands in sc->d_normal.  Queue sizes are read back once per level to
@@ -1195,6 +1200,7 @@ void ft_scene_destroy(ft_scene* sc) {
   cudaFree(sc->wf_shadows);
   cudaFree(sc->wf_primary_normal);
   cudaFree(sc->wf_counters);
+  cudaFree(sc->path_buf);
   for (cudaEvent_t e : sc->prof_pool) cudaEventDestroy(e);
   cudaSetDevice(prev);
   delete sc;
@@ -1313,10 +1319,30 @@ ft_status ft_render_pathtrace(ft_scene* sc, const ft_render_options* options, ft
   float* rgbf = rgb_out ? (dev_ptrs ? rgb_out : sc->d_rgbf) : nullptr;
   uint8_t* rgb8 = rgb8_out ? (dev_ptrs ? rgb8_out : sc->d_rgb) : nullptr;
   uint32_t* cnt = samples_out ? (dev_ptrs ? samples_out : sc->d_mat) : nullptr;
-  const unsigned blocks = static_cast<unsigned>((pixels + 127) / 128);
-  path_pixel_kernel<false><<<blocks, 128, 0, st>>>(sc->dev, P, ps, rgbf, rgb8, cnt, nullptr);
-  FT_CUDA_TRY(cudaGetLastError(), "path_pixel_kernel launch");
-  sc->last_launches = 1;
+  // Passes of samples: the first takes the min_spp that every pixel needs,
+  // later ones at most as many (samples behind a pixel's stop are wasted),
+  // bounded by the sample buffer.
+  const uint64_t cap = std::max<uint64_t>(1, kPathSamples / pixels);
+  const uint32_t most = static_cast<uint32_t>(
+      std::min<uint64_t>(cap, ps.noise_threshold > 0.0f ? std::max(ps.min_spp, 4u) : ps.spp));
+  const uint64_t floats = 3 * pixels * std::min(most, ps.spp) + pixels * (sizeof(PathPixel) / sizeof(float));
+  if (ft_status s = grow(&sc->path_buf, &sc->path_cap, floats, "cudaMalloc(path samples)")) return s;
+  auto* state = reinterpret_cast<PathPixel*>(sc->path_buf);
+  float* samples = sc->path_buf + pixels * (sizeof(PathPixel) / sizeof(float));
+  FT_CUDA_TRY(cudaMemsetAsync(state, 0, pixels * sizeof(PathPixel), st), "memset");
+  sc->last_launches = 0;
+  for (uint32_t first = 0; first < ps.spp;) {
+    const uint32_t n = std::min(ps.spp - first, most);
+    const uint64_t blocks = (pixels * n + 127) / 128;
+    path_sample_kernel<<<static_cast<unsigned>(blocks), 128, 0, st>>>(sc->dev, P, ps.max_bounces, first, n, state,
+                                                                      samples);
+    FT_CUDA_TRY(cudaGetLastError(), "path_sample_kernel launch");
+    first += n;
+    path_accumulate_kernel<<<static_cast<unsigned>((pixels + 127) / 128), 128, 0, st>>>(
+        pixels, ps, n, samples, state, first >= ps.spp ? 1 : 0, rgbf, rgb8, cnt);
+    FT_CUDA_TRY(cudaGetLastError(), "path_accumulate_kernel launch");
+    sc->last_launches += 2;
+  }
   if (!dev_ptrs) {
     if (rgb_out) FT_CUDA_TRY(cudaMemcpyAsync(rgb_out, rgbf, pixels * 3 * sizeof(float), cudaMemcpyDeviceToHost, st),
                              "copy rgb");
