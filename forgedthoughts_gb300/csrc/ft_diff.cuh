@@ -513,9 +513,10 @@ __device__ __noinline__ bool scene_backprop(const DevScene& S, F3 p, const DiffT
 //
 // One thread per ray to the end left a warp waiting for its longest search: a
 // miss takes 40 golden-section steps after its march, and an adjoint ray its
-// gradient.
+// gradient.  Eight blocks per SM (64 registers): 11.4 ms for the step above
+// against 12.4 with five.
 template <bool kAdjoint>
-__global__ void __launch_bounds__(128, 5) views_march_persistent(
+__global__ void __launch_bounds__(128, 8) views_march_persistent(
     const __grid_constant__ DevScene S, const RayParams* __restrict__ views, uint64_t items_per_view, uint64_t first,
     uint64_t n_work, float tau, float* __restrict__ t_out, uint8_t* __restrict__ mask_out, float* __restrict__ sil_out,
     const float* __restrict__ dl_dt, const float* __restrict__ dl_dsil, AdjointRay* __restrict__ records,

@@ -79,6 +79,7 @@ struct alignas(16) DevFast {
   int32_t tree_lhs;   // kFastTree: the tree is the BVH root's left child
   int32_t all;        // kFastUnion: every primitive is in the first n_always
   uint32_t entry[2];  // compact entries, kNoPrim for none
+  float4 rec[3];      // the compact record of entry[0], or of the first always-evaluated primitive
   float bmin[2][3], bmax[2][3];
   DevUrTree tree;
 };
@@ -778,6 +779,15 @@ __device__ __noinline__ Info scene_distance_general(const DevScene& S, F3 p, Ctx
   return scene_distance_leaves(S, p, leaf, second, second_lb, cx);
 }
 
+// The primitive of DevFast::rec (a ground, usually), from the constant bank.
+template <bool kSphereYX, bool kStats>
+__device__ __forceinline__ float fast_prim(const DevScene& S, F3 p, Ctx<kStats>& cx) {
+  cx.prim();
+  const float4* w = S.fast.rec;
+  if (__float_as_uint(w[2].w) & ftd::kRareFlag) return rare_distance(S.nodes[__float_as_int(w[2].z)], p);
+  return ftd::compact_distance<kSphereYX>(w[0], w[1], w[2].x, w[2].y, p);
+}
+
 __device__ __forceinline__ int32_t compact_ref(uint32_t entry) { return ~static_cast<int32_t>(entry & ~ftd::kRareFlag); }
 
 // kFastTree with a primitive leaf: the two-leaf walk above (nearer box first,
@@ -791,7 +801,7 @@ template <bool kStats>
 __device__ __forceinline__ Info tree_and_prim(const DevScene& S, F3 p, float t2, float p2, Ctx<kStats>& cx) {
   const DevFast& F = S.fast;
   const bool tree_first = F.tree_lhs ? t2 <= p2 : t2 < p2;
-  const Info prim{compact_at(S, F.entry[0], p, cx), compact_ref(F.entry[0])};
+  const Info prim{fast_prim<false>(S, p, cx), compact_ref(F.entry[0])};
   if (!tree_first && !(sqrtf(t2) <= prim.d)) return prim;
   const Info tree = eval_urtree(S, F.tree, p, tree_first && prim.d < 0.0f ? kInf : prim.d, cx);
   if (!tree_first) return tree.d < prim.d ? tree : prim;
@@ -833,8 +843,9 @@ __device__ __forceinline__ Info union_distance(const DevScene& S, F3 p, Ctx<kSta
     if (d < best.d) best = Info{d, ~i};
     negative += d < 0.0f;
   };
-#pragma unroll 4
-  for (int i = 0; i < F.n_always; ++i) {  // the same record for every lane
+  if (F.n_always > 0) add(fast_prim<true>(S, p, cx), 0);
+#pragma unroll 1
+  for (int i = 1; i < F.n_always; ++i) {  // the same record for every lane
     const float4* w = S.cprims + 3 * i;
     const float4 a = __ldg(w), b = __ldg(w + 1), c = __ldg(w + 2);
     cx.prim();
@@ -993,14 +1004,27 @@ __device__ HitOut march(const DevScene& S, const RayParams& P, F3 o, F3 d, bool 
   return h;
 }
 
+// Pixel and sample of work item i.  32-bit divisions where the frame allows: a
+// 64-bit one is a call of some hundred instructions, in the refill that a warp
+// of the persistent marches runs for a few lanes at a time.
 __device__ __forceinline__ void item_coords(const RayParams& P, uint64_t i, uint32_t* px, uint32_t* py, uint32_t* s) {
-  uint32_t per_tile = P.tile_w * P.tile_h * P.aa;
-  uint64_t tile = i / per_tile;
-  uint32_t k = static_cast<uint32_t>(i - tile * per_tile);
+  const uint32_t per_tile = P.tile_w * P.tile_h * P.aa;
+  uint32_t k, tx, ty;
+  if (P.n_items <= 0xffffffffull) {
+    const uint32_t i32 = static_cast<uint32_t>(i), tile = i32 / per_tile;
+    k = i32 - tile * per_tile;
+    ty = tile / P.tiles_x;
+    tx = tile - ty * P.tiles_x;
+  } else {
+    const uint64_t tile = i / per_tile;
+    k = static_cast<uint32_t>(i - tile * per_tile);
+    tx = static_cast<uint32_t>(tile % P.tiles_x);
+    ty = static_cast<uint32_t>(tile / P.tiles_x);
+  }
   *s = k % P.aa;
-  uint32_t j = k / P.aa;
-  *px = static_cast<uint32_t>(tile % P.tiles_x) * P.tile_w + j % P.tile_w;
-  *py = static_cast<uint32_t>(tile / P.tiles_x) * P.tile_h + j / P.tile_w;
+  const uint32_t j = k / P.aa;
+  *px = tx * P.tile_w + j % P.tile_w;
+  *py = ty * P.tile_h + j / P.tile_w;
 }
 
 #include "ft_bricks.cuh"
@@ -1120,10 +1144,10 @@ constexpr unsigned long long kMarchWallNs = 20ull * 1000000000ull;  // per warp
 // brick cache from the batch tables (otherwise they are the kernel's own
 // parameters); outputs are the concatenated arrays of all items.
 //
-// Five resident blocks per SM (at most 102 registers): measured on the
-// 512-primitive field at 1920x1080, 167 Mrays/s against 165 with six blocks
-// (80 registers), 161 with four, 148 with the compiler's own choice (64
-// registers and more spills) and 132 with one block (123 registers).
+// Five resident blocks per SM (96 registers): a small frame is bound by the
+// latency of its longest rays' evaluations and a 256x256 preview takes 0.42 ms
+// of march against 0.46 with six or eight blocks; the 512-primitive field at
+// 1920x1080 takes 12.7, 12.7 and 11.8 ms (refilling at 8 idle lanes).
 template <bool kStats, bool kBricks, bool kBatch>
 __global__ void __launch_bounds__(128, 5) march_depth_persistent(
     const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ DevBricks B0,

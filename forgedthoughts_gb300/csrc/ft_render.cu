@@ -527,6 +527,8 @@ ft_status upload_scene(ft_scene* sc) {
       for (size_t k = 0; k < jobs.size(); ++k) (k == 0 ? F.tree.fine : F.tree.outer) = dev_grid(jobs[k]);
     }
   }
+  if (F.kind == kFastUnion || (F.kind == kFastTree && F.entry[0] != kNoPrim))
+    std::memcpy(F.rec, &cprims[F.kind == kFastUnion ? 0 : F.entry[0] & ~ftd::kRareFlag], sizeof(F.rec));
   // [0, 8): statistics counters; [8]: work-item counter of the persistent march
   FT_CUDA_TRY(cudaMalloc(&sc->d_stats, kStatWords * sizeof(unsigned long long)), "cudaMalloc(stats)");
   int sms = 0, per_sm = 0;
@@ -608,7 +610,7 @@ RayParams make_params(const ft_scene* sc, const ft_render_options& o, uint32_t a
   P.eps = o.epsilon;
   P.step_scale = o.step_scale;
   set_tiles(&P, 8, 4);
-  P.refill = 8;
+  P.refill = 24;
   P.jitter = 0;
   P.jitter_seed = 0;
   return P;
@@ -741,7 +743,7 @@ struct ft_batch {
   // they never touch them under a launch still running on another stream.
   cudaEvent_t done = nullptr;
   cudaGraphExec_t exec = nullptr;
-  ft_batch_tuning tuning{8, 8, 8, 0.0f};
+  ft_batch_tuning tuning{8, 8, 24, 0.0f};
   std::mutex mu;
   // Wavefront queues of the trace items (sized per tuning: tiles pad the
   // work items), their counters (job counts x2, shadow count, overflow
@@ -2033,9 +2035,9 @@ std::vector<RayParams> view_params(const ft_scene* sc, const ft_view* views, uin
 // Rays of one pass of the adjoint (24 bytes of records each).
 constexpr uint64_t kAdjointChunk = uint64_t(1) << 22;
 
-// Blocks of a views pass over n rays: five per SM, its resident blocks.
+// Blocks of a views pass over n rays: eight per SM, its resident blocks.
 unsigned view_blocks(const ft_scene* sc, uint64_t n) {
-  const uint64_t resident = static_cast<uint64_t>(sc->sms) * 5;
+  const uint64_t resident = static_cast<uint64_t>(sc->sms) * 8;
   return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n + 127) / 128, resident)));
 }
 

@@ -148,8 +148,15 @@ __device__ __forceinline__ void wf_shade_job(const DevScene& S, const RayParams&
        i < (n); i += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
 
 // With kStats the kernel sums its work counters into stats[0 .. kNumCounters).
+// Bound by instruction fetch: a hit runs thousands of instructions once
+// (no_instruction is half of the stalls).  Left at the compiler's four blocks
+// per SM and with the hook interpreter inlined: six blocks take 86 ms against
+// 91 for the 512-primitive field's frame and the interpreter out of line 81,
+// but either contracts a hook's multiply-adds otherwise, and hooked scenes,
+// whose normals difference values 1e-4 apart, change.
 template <bool kStats>
-__global__ void __launch_bounds__(128) wf_shade_kernel(const __grid_constant__ DevScene S, const __grid_constant__ RayParams P, const WJob* __restrict__ jobs,
+__global__ void __launch_bounds__(128) wf_shade_kernel(const __grid_constant__ DevScene S,
+                                                          const __grid_constant__ RayParams P, const WJob* __restrict__ jobs,
                                                        const unsigned long long* __restrict__ count,
                                                        unsigned long long cap, const WHit* __restrict__ hits,
                                                        WQueues Q, unsigned long long* __restrict__ stats) {
@@ -180,12 +187,15 @@ __device__ __forceinline__ uint32_t sample_item(const BatchView& V, uint64_t sam
 // job to the end, so a warp waits for its longest march (the shadow kernel
 // kept 8 of 32 lanes busy).  Here every lane runs one distance evaluation per
 // iteration of a small state machine and takes the next job of the queue
-// (one atomic per warp) once at least kWfRefill lanes are idle.  With kBatch
+// (one atomic per warp) once at least kWfRefill lanes are idle: setting up a
+// ray is several hundred instructions whose cost the waiting lanes share, so
+// few large refills beat keeping the lanes full (1920x1080 depth of the
+// 512-primitive field: 14.8 ms at 4, 12.7 at 8, 12.0 at 16, 11.1 at 24).  With kBatch
 // each job's render (scene, parameters) is looked up from its sample index.
 // Self-checks as in march_depth_persistent: a job may take at most
 // max_steps + 64 iterations, a warp at most kMarchWallNs; a lane past either
 // limit sets a bit in *flags and gives up.
-constexpr unsigned kWfRefill = 8;
+constexpr unsigned kWfRefill = 24;
 
 #define FT_WF_REFILL_TOP(live, queue_done, n_jobs, next_job, base_out, took)                       \
   if ((++loop_iters & 1023u) == 0u) {                                                            \
@@ -230,7 +240,8 @@ __device__ __noinline__ void wf_add_miss(const DevScene& S, const RayParams& P, 
 // hit leaf's lookup (march_hit, one evaluation per iteration); a miss adds
 // the environment seen through the ray's medium.  Five resident blocks per SM
 // (the launch is five per SM): on the 512-primitive field's depth-6 trace,
-// 181 ms of march per frame against 185 with six and 195 with four.
+// 70 ms of march per frame against 73 with six and 71 with eight, and a
+// 353x199 trace, bound by its longest rays' latency, 2.0 against 2.2 ms.
 template <bool kBatch, bool kStats>
 __global__ void __launch_bounds__(128, 5) wf_march_persistent(
     const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ BatchView V,
