@@ -349,7 +349,7 @@ ft_status upload_scene(ft_scene* sc) {
     d.fallback_first = t.fallback_first;
     d.fallback_count = t.fallback_count;
     d.far_first = static_cast<int32_t>(far_nodes.size());
-    ftgpu::build_far_tree(im, im.cprims, t.prim_first, t.n_prims, &far_nodes, &far_entries);
+    if (t.dims[0] > 0) ftgpu::build_far_tree(im, im.cprims, t.prim_first, t.n_prims, &far_nodes, &far_entries);
     d.far_end = static_cast<int32_t>(far_nodes.size());
     trees.push_back(d);
   }
@@ -527,6 +527,9 @@ ft_status upload_scene(ft_scene* sc) {
       for (size_t k = 0; k < jobs.size(); ++k) (k == 0 ? F.tree.fine : F.tree.outer) = dev_grid(jobs[k]);
     }
   }
+  // (without any grid the far walk would meet points inside the solids, where
+  // the leaf walk's order counts)
+  if (F.kind == kFastUnion && !F.all && F.tree.fine.dims[0] <= 0 && F.tree.outer.dims[0] <= 0) F.kind = kFastNone;
   if (F.kind == kFastUnion || (F.kind == kFastTree && F.entry[0] != kNoPrim))
     std::memcpy(F.rec, &cprims[F.kind == kFastUnion ? 0 : F.entry[0] & ~ftd::kRareFlag], sizeof(F.rec));
   // [0, 8): statistics counters; [8]: work-item counter of the persistent march

@@ -845,6 +845,8 @@ class Builder {
   // radius), which stay on the tree BVH.
   bool sane_prim(const HostNode& n) const {
     const float* f = n.f;
+    for (int a = 0; a < 3; ++a)
+      if (!std::isfinite(n.c[a]) || !std::isfinite(n.bmin[a]) || !std::isfinite(n.bmax[a])) return false;
     switch (n.kind) {
       case FT_NODE_SPHERE: return f[0] >= 0.0f;
       case FT_NODE_BOX:
