@@ -116,22 +116,23 @@ __global__ void __launch_bounds__(64) grid_cells_kernel(const __grid_constant__ 
   const F3 m = f3(J.gmin[0] + (x + 0.5f) * J.cell, J.gmin[1] + (y + 0.5f) * J.cell, J.gmin[2] + (z + 0.5f) * J.cell);
   float limit = 0.0f;
   unsigned count = 0;
-  if (mine) {
+  if (mine && kFill) {
+    // the count pass left the cell's limit beside its count
+    const uint2 c = cells[cell];
+    limit = __uint_as_float(c.x);
+    count = c.y;
+    if (count == kInsideCell) {
+      count = 0;
+      mine = false;
+    }
+  } else if (mine) {
     float best = kInf;
     for (int k = 0; k < n; ++k) best = fminf(best, grid_bound(S, J.prim_first + (all ? k : keep[k]), m, half).d);
     limit = fmaxf(J.r, best + half * 1.7320509f) + J.slack;
-    if (kFill) {
-      count = cells[cell].y;
-      if (count == kInsideCell) {
-        count = 0;
-        mine = false;
-      }
-    } else {
-      const bool inside = J.skip_inside && best + half * 1.7320509f < -J.slack;
-      for (int k = 0; k < (inside ? 0 : n); ++k)
-        count += grid_bound(S, J.prim_first + (all ? k : keep[k]), m, half).low - J.slack < limit;
-      cells[cell] = make_uint2(0u, inside ? kInsideCell : count);
-    }
+    const bool inside = J.skip_inside && best + half * 1.7320509f < -J.slack;
+    for (int k = 0; k < (inside ? 0 : n); ++k)
+      count += grid_bound(S, J.prim_first + (all ? k : keep[k]), m, half).low - J.slack < limit;
+    cells[cell] = make_uint2(__float_as_uint(limit), inside ? kInsideCell : count);
   }
   // the block's entries: counted into the total, or allocated from it
   unsigned scan = count;
