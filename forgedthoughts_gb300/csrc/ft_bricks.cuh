@@ -59,7 +59,7 @@ __device__ Info scene_distance_skip(const DevScene& S, F3 p, const DevBricks& B,
     bool skip = false;
     for (int i = 0; i < B.n_exact; ++i) skip |= (B.exact_leaf[i] == leaf);
     if (skip) continue;
-    const Info in = eval_leaf(S, S.leaves[leaf], p, cur.d, cx);
+    const Info in = eval_leaf(S, leaf, p, cur.d, cx);
     if (in.d < cur.d) cur = in;
   }
   return cur;
@@ -78,7 +78,7 @@ __device__ __forceinline__ bool far_bound(const DevScene& S, const DevBricks& B,
   cx.fetch();
   // texel centres sit at integer + 0.5 in unnormalised coordinates
   float v = tex3D<float>(B.atlas, gx + 0.5f, gy + 0.5f, gz + 0.5f);
-  for (int i = 0; i < B.n_exact; ++i) v = fminf(v, eval_leaf(S, S.leaves[B.exact_leaf[i]], p, kInf, cx).d);
+  for (int i = 0; i < B.n_exact; ++i) v = fminf(v, eval_leaf(S, B.exact_leaf[i], p, kInf, cx).d);
   *out = v;
   return true;
 }

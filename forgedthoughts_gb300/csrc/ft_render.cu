@@ -399,13 +399,32 @@ ft_status upload_scene(ft_scene* sc) {
   }
   // Leaves with their device kinds: [distance_post] [domain] primitive
   std::vector<ftgpu::HostLeaf> leaves = im.leaves;
+  std::vector<float4> hooked;
   for (ftgpu::HostLeaf& l : leaves) {
     if (l.kind != ftgpu::kLeafGeneric) continue;
-    int32_t k = l.node;
-    if (im.nodes[k].kind == FT_NODE_DISTANCE_POST) k = im.nodes[k].a;
-    if (im.nodes[k].kind == FT_NODE_DOMAIN) k = im.nodes[k].a;
-    if (k != l.node && im.nodes[k].kind <= FT_NODE_EXTRUDE_POLYGON) l.kind = ftgpu::kLeafHooked;
+    const int32_t post = im.nodes[l.node].kind == FT_NODE_DISTANCE_POST ? l.node : -1;
+    const int32_t below = post >= 0 ? im.nodes[post].a : l.node;
+    const int32_t dom = im.nodes[below].kind == FT_NODE_DOMAIN ? below : -1;
+    const int32_t prim = dom >= 0 ? im.nodes[dom].a : below;
+    if ((post < 0 && dom < 0) || im.nodes[prim].kind > FT_NODE_EXTRUDE_POLYGON) continue;
+    l.kind = ftgpu::kLeafHooked;
+    l.first = -1;
+    const ftgpu::CompactPrim c = ftgpu::compact_prim(im, prim, static_cast<uint32_t>(&l - leaves.data()));
+    if ((c.leaf & ftd::kRareFlag) || (post >= 0 && im.nodes[post].has_rot) || (dom >= 0 && im.nodes[dom].has_rot))
+      continue;
+    l.first = static_cast<int32_t>(hooked.size() / kHookedWords);
+    for (int32_t k : {post, dom}) {
+      float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const int32_t program = k >= 0 ? im.nodes[k].program : -1;
+      if (k >= 0) w = make_float4(im.nodes[k].c[0], im.nodes[k].c[1], im.nodes[k].c[2], 0.0f);
+      std::memcpy(&w.w, &program, sizeof(w.w));
+      hooked.push_back(w);
+    }
+    hooked.resize(hooked.size() + kHookedWords - 2);
+    std::memcpy(&hooked[hooked.size() - (kHookedWords - 2)], &c, sizeof(c));
   }
+  std::vector<int4> leaf_info;
+  for (const ftgpu::HostLeaf& l : leaves) leaf_info.push_back(make_int4(l.kind, l.node, l.first, l.count));
   std::vector<Part> parts;
   auto part = [&](const void* src, size_t bytes) {
     parts.push_back(Part{src, bytes, 0});
@@ -418,7 +437,8 @@ ft_status upload_scene(ft_scene* sc) {
                p_instrs = vec(im.instrs), p_cprims = vec(cprims), p_paths = vec(im.ur_paths),
                p_materials = vec(im.materials), p_lights = vec(im.lights), p_op_begin = vec(im.node_op_begin),
                p_op_end = vec(im.node_op_end), p_blend = vec(im.ur_inner_blend), p_obj = vec(im.obj_node),
-               p_far = vec(far_nodes), p_far_entries = vec(far_entries), p_pairs = vec(pairs);
+               p_far = vec(far_nodes), p_far_entries = vec(far_entries), p_pairs = vec(pairs), p_info = vec(leaf_info),
+               p_hooked = vec(hooked);
   size_t total = 0;
   for (Part& p : parts) {
     p.off = total;
@@ -456,6 +476,8 @@ ft_status upload_scene(ft_scene* sc) {
   at(p_obj, d.obj_node);
   at(p_far, d.far_nodes);
   at(p_pairs, d.bvh_pairs);
+  at(p_info, d.leaf_info);
+  at(p_hooked, d.hooked);
   d.bvh_ref = bvh_ref(im.bvh_root);
   at(p_far_entries, d.far_entries);
   d.n_obj_node = static_cast<int32_t>(im.obj_node.size());

@@ -53,6 +53,25 @@ bool is_unary(int k) {
 
 float deg_to_rad(float d) { return d * (3.14159265358979323846f / 180.0f); }
 
+// Whether a primitive's distance is 1-Lipschitz and at least its box's: what
+// the candidate grids and the box culling rest on.  The parser's shapes are;
+// a node record may hold others (a rounding above the half size, a negative
+// radius), which stay on the tree BVH.
+bool sane_prim(const HostNode& n) {
+  const float* f = n.f;
+  for (int a = 0; a < 3; ++a)
+    if (!std::isfinite(n.c[a]) || !std::isfinite(n.bmin[a]) || !std::isfinite(n.bmax[a])) return false;
+  switch (n.kind) {
+    case FT_NODE_SPHERE: return f[0] >= 0.0f;
+    case FT_NODE_BOX:
+      return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[3] >= 0.0f && f[3] <= std::min(f[0], std::min(f[1], f[2]));
+    case FT_NODE_CYLINDER: return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[2] <= std::min(f[0], f[1]);
+    case FT_NODE_TORUS: return f[0] >= 0.0f && f[1] >= 0.0f;
+    default: return false;
+  }
+}
+
+
 class Builder {
  public:
   Builder(const ft_scene_desc& d, SceneImage* img, std::string* err, bool lists)
@@ -122,14 +141,14 @@ class Builder {
       } else if (lv[1 - k].kind == kLeafPrim) {
         img_->fast_tree = k;
         img_->fast_prim = 1 - k;
-        img_->cprims.push_back(compact_prim(lv[1 - k].node, lv[1 - k]));
+        img_->cprims.push_back(compact_prim(*img_, lv[1 - k].node, leaf_index(lv[1 - k])));
       }
     }
     img_->fast_union = std::all_of(lv.begin(), lv.end(), [&](const HostLeaf& l) {
       return l.kind == kLeafPrim && sane_prim(img_->nodes[l.node]);
     });
     if (img_->fast_union)
-      for (const HostLeaf& l : lv) img_->cprims.push_back(compact_prim(l.node, l));
+      for (const HostLeaf& l : lv) img_->cprims.push_back(compact_prim(*img_, l.node, leaf_index(l)));
     return true;
   }
 
@@ -839,44 +858,7 @@ class Builder {
     return true;
   }
 
-  // Whether a primitive's distance is 1-Lipschitz and at least its box's: what
-  // the candidate grids and the box culling rest on.  The parser's shapes are;
-  // a node record may hold others (a rounding above the half size, a negative
-  // radius), which stay on the tree BVH.
-  bool sane_prim(const HostNode& n) const {
-    const float* f = n.f;
-    for (int a = 0; a < 3; ++a)
-      if (!std::isfinite(n.c[a]) || !std::isfinite(n.bmin[a]) || !std::isfinite(n.bmax[a])) return false;
-    switch (n.kind) {
-      case FT_NODE_SPHERE: return f[0] >= 0.0f;
-      case FT_NODE_BOX:
-        return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[3] >= 0.0f && f[3] <= std::min(f[0], std::min(f[1], f[2]));
-      case FT_NODE_CYLINDER: return f[0] >= 0.0f && f[1] >= 0.0f && f[2] >= 0.0f && f[2] <= std::min(f[0], f[1]);
-      case FT_NODE_TORUS: return f[0] >= 0.0f && f[1] >= 0.0f;
-      default: return false;
-    }
-  }
-
-  CompactPrim compact_prim(int node, const HostLeaf& leaf) const {
-    const HostNode& n = img_->nodes[node];
-    CompactPrim c;
-    std::memset(&c, 0, sizeof(c));
-    std::memcpy(c.c, n.c, sizeof(c.c));
-    c.node = node;
-    c.leaf = static_cast<uint32_t>(&leaf - img_->leaves.data());
-    const bool y_only = !n.has_rot || (d_.nodes[node].rot_deg[0] == 0.0f && d_.nodes[node].rot_deg[2] == 0.0f);
-    if (!y_only || (n.kind != FT_NODE_SPHERE && n.kind != FT_NODE_BOX) || !sane_prim(n)) {
-      c.leaf |= 0x80000000u;
-      return c;
-    }
-    c.cos = n.has_rot ? n.cy : 1.0f;
-    c.sin = n.has_rot ? n.sy : 0.0f;
-    const float shell = n.kind == FT_NODE_SPHERE ? n.f[1] : n.f[4];
-    c.shell = shell > 0.0f ? shell : std::numeric_limits<float>::infinity();
-    c.rd = n.kind == FT_NODE_SPHERE ? n.f[0] : n.f[3];
-    for (int a = 0; a < 3; ++a) c.h[a] = n.kind == FT_NODE_SPHERE ? 0.0f : std::max(n.f[a] - n.f[3], 0.0f);
-    return c;
-  }
+  uint32_t leaf_index(const HostLeaf& l) const { return static_cast<uint32_t>(&l - img_->leaves.data()); }
 
   bool build_urtree(HostLeaf& leaf, float r, int depth) {
     HostUrTree t;
@@ -906,7 +888,7 @@ class Builder {
     // Compact records and root paths (the device folds near primitives along
     // them).
     for (int32_t i : std::vector<int32_t>(img_->ur_prims.begin() + t.prim_first, img_->ur_prims.end()))
-      img_->cprims.push_back(compact_prim(i, leaf));
+      img_->cprims.push_back(compact_prim(*img_, i, leaf_index(leaf)));
     img_->ur_paths.resize(img_->ur_prims.size(), UrPath{0, 0, 0});
     std::function<void(int, uint64_t, uint32_t)> paths = [&](int c, uint64_t sides, uint32_t dep) {
       if (c < 0) {
@@ -962,6 +944,27 @@ class Builder {
 };
 
 }  // namespace
+
+CompactPrim compact_prim(const SceneImage& img, int node, uint32_t leaf) {
+  const HostNode& n = img.nodes[node];
+  CompactPrim c;
+  std::memset(&c, 0, sizeof(c));
+  std::memcpy(c.c, n.c, sizeof(c.c));
+  c.node = node;
+  c.leaf = leaf;
+  const bool y_only = !n.has_rot || (n.sx == 0.0f && n.cx == 1.0f && n.sz == 0.0f && n.cz == 1.0f);
+  if (!y_only || (n.kind != FT_NODE_SPHERE && n.kind != FT_NODE_BOX) || !sane_prim(n)) {
+    c.leaf |= 0x80000000u;
+    return c;
+  }
+  c.cos = n.has_rot ? n.cy : 1.0f;
+  c.sin = n.has_rot ? n.sy : 0.0f;
+  const float shell = n.kind == FT_NODE_SPHERE ? n.f[1] : n.f[4];
+  c.shell = shell > 0.0f ? shell : std::numeric_limits<float>::infinity();
+  c.rd = n.kind == FT_NODE_SPHERE ? n.f[0] : n.f[3];
+  for (int a = 0; a < 3; ++a) c.h[a] = n.kind == FT_NODE_SPHERE ? 0.0f : std::max(n.f[a] - n.f[3], 0.0f);
+  return c;
+}
 
 bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error, bool lists) {
   *out = SceneImage{};

@@ -138,6 +138,10 @@ struct SceneImage {
 // scene on a device builds its own lists there.
 bool build_scene_image(const ft_scene_desc& desc, SceneImage* out, std::string* error, bool lists);
 
+// Compact record of a primitive node (rare-flagged where its kind or turn has
+// none).
+CompactPrim compact_prim(const SceneImage& img, int node, uint32_t leaf);
+
 // Tree over compact primitives for points outside their candidate grids, in
 // depth-first order: a walk goes to the next node, or past a subtree whose box
 // is out of reach, and needs no stack.
