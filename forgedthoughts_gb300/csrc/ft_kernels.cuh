@@ -1149,9 +1149,10 @@ __device__ __forceinline__ bool item_ray(const RayParams& P, uint64_t i, F3* dir
 // live lane, whatever the lane is doing: a march step (R:4100-4137), one of
 // the ten bisection steps (refine_hit_distance, R:4180-4200), one of the six
 // estimate_normal taps (R:4202-4215) or the final material lookup.  Lanes
-// whose ray finished pick up the next work item from a global counter once a
-// quarter of the warp is idle, so divergent march lengths do not leave lanes
-// idle for the rest of the warp's life.  The sequence of evaluation points of
+// whose ray finished pick up the next work item from a global counter once
+// `refill` lanes of the warp are idle (24 by default: see kWfRefill), so
+// divergent march lengths do not leave lanes idle for the rest of the warp's
+// life.  The sequence of evaluation points of
 // each ray is exactly the reference's.
 //
 // With kBricks (the FP16 precision form) a ray starts in the far-field phase:
