@@ -67,7 +67,8 @@ struct DevUrInner {
 // the general leaf walk; its data are kernel parameters, read from the constant
 // bank.
 //   kFastTree   one union_round tree (`tree`, box 1), alone or beside one
-//               primitive (entry[0], box 0);
+//               primitive whose distance is at least its box's (entry[0],
+//               box 0; an extruded polygon's is not);
 //   kFastPair   two primitives (entry and boxes 0, 1: the BVH root's children);
 //   kFastUnion  primitives only: the first n_always compact records at every
 //               point, the others through the candidate grids and far walk of

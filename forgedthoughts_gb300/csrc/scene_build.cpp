@@ -138,7 +138,9 @@ class Builder {
       if (lv[k].kind != kLeafUrTree) continue;
       if (lv.size() == 1) {
         img_->fast_tree = k;
-      } else if (lv[1 - k].kind == kLeafPrim) {
+      } else if (lv[1 - k].kind == kLeafPrim && sane_prim(img_->nodes[lv[1 - k].node])) {
+        // (its distance bounds the tree's walk, so it must be at least its
+        // box's: an extruded polygon's is not)
         img_->fast_tree = k;
         img_->fast_prim = 1 - k;
         img_->cprims.push_back(compact_prim(*img_, lv[1 - k].node, leaf_index(lv[1 - k])));

@@ -103,8 +103,8 @@ struct SceneImage {
   // per ur_cell_prims entry: a lower bound of the distance from any point of
   // the cell to the primitive's box (the lists are sorted by it)
   std::vector<float> ur_cell_gaps;
-  // A scene of one union_round tree, alone or beside one primitive: their
-  // leaves, -1 for other scenes (and no primitive).
+  // A scene of one union_round tree, alone or beside one primitive whose box
+  // bounds its distance: their leaves, -1 for other scenes (and no primitive).
   int32_t fast_tree = -1, fast_prim = -1;
   // All leaves are primitives whose boxes bound their distances.
   bool fast_union = false;

@@ -1,0 +1,78 @@
+"""Where the short scene forms, the candidate grids, the material resolve, the
+views passes and the path tracer's passes reach their limits: primitives whose
+distance is not bounded by their box, hits that lie farther from the surface
+than the blend radius, scenes of very many trees, marches of unbounded length,
+large sample counts, ties."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import forgedthoughts_gb300 as ft
+import oracle
+from forgedthoughts_gb300 import _native, workloads
+
+pytestmark = pytest.mark.gpu
+
+LIGHTS = ("let camera = Camera { origin: vec3(0, 1.2, -5), target: vec3(0, 0.6, 0), fov_y: 45.0 };\n"
+          "let light = PointLight { position: vec3(3, 6, -3), intensity: 60.0 };\n")
+
+
+def _points(n, reach, seed=11):
+    rng = np.random.default_rng(seed)
+    return rng.uniform([-reach, -0.5 * reach, -reach], [reach, reach, reach], size=(n, 3)).astype(np.float32)
+
+
+def _distances(st, pts):
+    g = st.gpu()
+    g.build_bricks(0.25)
+    return g.brick_bounds(pts)[1].astype(np.float64)
+
+
+def _tree(names, k, tag="u"):
+    """A balanced pairwise union_round(k) tree: its lines and its root."""
+    lines, cur, level = [], list(names), 0
+    while len(cur) > 1:
+        nxt = []
+        for j in range(0, len(cur) - 1, 2):
+            lines.append(f"let {tag}{level}_{j // 2} = {cur[j]}.union_round({cur[j + 1]}, {k});")
+            nxt.append(f"{tag}{level}_{j // 2}")
+        cur, level = nxt + cur[len(cur) - len(cur) % 2:], level + 1
+    return lines, cur[0]
+
+
+SPHERES = [f"let s{i} = Sphere {{ radius: 0.3, pos: vec3({x}, 0.5, {z}) }};"
+           for i, (x, z) in enumerate([(-2.2, -1.9), (1.7, -2.1), (-1.8, 2.0), (2.1, 1.6)])]
+
+
+@pytest.mark.parametrize("tree_first", [False, True])
+@pytest.mark.parametrize("sides", [3, 6])
+def test_tree_beside_an_extruded_polygon(sides, tree_first):
+    """An extruded polygon's distance is measured to its edge lines and can be
+    less than its box's, so it must not bound the walk of a tree beside it.
+    Tolerance as for the other distances of a scene: 1e-5 of the value or 1."""
+    lines, root = _tree([f"s{i}" for i in range(4)], 0.3)
+    prism = f"let prism = ExtrudePolygon {{ sides: {sides}, radius: 1.0, height: 0.6, pos: vec3(0.3, 0.4, -0.2) }};"
+    src = "\n".join(SPHERES + lines + [prism]) + "\nlet scene = " + (
+        f"{root} + prism;\n" if tree_first else f"prism + {root};\n")
+    st = ft.parse_and_eval(src)
+    pts = _points(60000, 9.0)
+    ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
+    err = np.abs(_distances(st, pts) - ref)
+    # (which leaf the walk visits hangs on comparisons of box bounds: a point
+    # within a rounding step of one may go either way)
+    assert (err > 1e-5 * np.maximum(1.0, np.abs(ref))).sum() <= 2, (float(err.max()), pts[err.argmax()])
+
+
+def test_tree_beside_a_box_rounded_past_its_size():
+    """A node record may hold a rounding above the half size; its box does not
+    bound its distance either."""
+    lines, root = _tree([f"s{i}" for i in range(4)], 0.3)
+    src = "\n".join(SPHERES + lines + ["let b = Box { size: vec3(0.4, 0.4, 0.4), round: 0.1, pos: vec3(0, 0.6, 0) };"])
+    st = ft.parse_and_eval(src + f"\nlet scene = {root} + b;\n")
+    box = [i for i in range(st.desc.n_nodes) if st.desc.nodes[i].kind == _native.FT_NODE_BOX]
+    ctypes.cast(st.desc.nodes, ctypes.POINTER(_native.NodeC))[box[0]].f[3] = 0.9
+    pts = _points(60000, 9.0)
+    ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
+    err = np.abs(_distances(st, pts) - ref)
+    assert (err > 1e-5 * np.maximum(1.0, np.abs(ref))).sum() <= 2, (float(err.max()), pts[err.argmax()])
