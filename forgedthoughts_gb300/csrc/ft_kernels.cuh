@@ -828,8 +828,9 @@ __device__ __forceinline__ int32_t compact_ref(uint32_t entry) { return ~static_
 // primitive evaluated first in either order, so that its distance bounds the
 // tree's walk.  t2 and p2 are the squared box bounds of the tree and the
 // primitive.  Where the tree comes first it is exact below the cutoff, and at
-// or above it the primitive's distance wins as it would there; a negative
-// primitive distance (a point inside it) does not cut the walk.
+// or above it the primitive's distance wins as it would there (a walk outside
+// the grids that finds nothing below the cutoff returns it without a surface);
+// a negative primitive distance (a point inside it) does not cut the walk.
 template <bool kStats>
 __device__ __forceinline__ Info tree_and_prim(const DevScene& S, F3 p, float t2, float p2, Ctx<kStats>& cx) {
   const DevFast& F = S.fast;
@@ -838,7 +839,7 @@ __device__ __forceinline__ Info tree_and_prim(const DevScene& S, F3 p, float t2,
   if (!tree_first && !(sqrtf(t2) <= prim.d)) return prim;
   const Info tree = eval_urtree(S, F.tree, p, tree_first && prim.d < 0.0f ? kInf : prim.d, cx);
   if (!tree_first) return tree.d < prim.d ? tree : prim;
-  return prim.d < tree.d && sqrtf(p2) <= tree.d ? prim : tree;
+  return tree.ref == ftd::kNoRef || (prim.d < tree.d && sqrtf(p2) <= tree.d) ? prim : tree;
 }
 
 // kFastPair: the two-leaf walk of two primitives.

@@ -76,3 +76,22 @@ def test_tree_beside_a_box_rounded_past_its_size():
     ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
     err = np.abs(_distances(st, pts) - ref)
     assert (err > 1e-5 * np.maximum(1.0, np.abs(ref))).sum() <= 2, (float(err.max()), pts[err.argmax()])
+
+
+def test_material_of_a_primitive_nearer_than_the_tree():
+    """A hit (of a large epsilon) on the primitive beside a tree, at a point
+    outside the tree's grids where the tree's box is the nearer one: the
+    tree's walk ends without a surface below the primitive's distance, and the
+    hit carries the primitive's material."""
+    lines = [f"let s{i} = Sphere {{ radius: 0.01, pos: vec3({x}, {y}, 0.0), material: Metal {{ roughness: 0.1 }} }};"
+             for i, (x, y) in enumerate([(-0.05, -1.5), (0.05, -1.5), (-0.05, 1.5), (0.05, 1.5)])]
+    ups, root = _tree([f"s{i}" for i in range(4)], 0.01)
+    ball = "let ball = Sphere { radius: 0.1, pos: vec3(0, 0, -3.6), material: Lambert { color: vec3(1, 0, 0) } };"
+    camera = "let camera = Camera { origin: vec3(-6, 0, -1.7), target: vec3(0, 0, -1.7), fov_y: 3.0 };"
+    st = ft.parse_and_eval("\n".join(lines + ups + [ball, camera]) + f"\nlet scene = {root} + ball;\n")
+    opts = ft.RenderOptions(width=64, height=64, max_steps=64, max_dist=20.0, epsilon=1.85, step_scale=0.5)
+    img = ft.render_depth(st, opts, ft.AccelMode.Bvh, 1, want_material=True)
+    _, m, mat, _, _ = oracle.render_depth(st, opts, 1, 1, 32)
+    both = (img.mask == 1) & (m == 1)
+    assert both.mean() > 0.5 and (mat[both] != 0).all()
+    assert (img.material[both] == mat[both]).all()
