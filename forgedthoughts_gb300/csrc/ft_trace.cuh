@@ -716,6 +716,10 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
     *need = -1.0f;
     return false;
   }
+  if (ng == 0) {  // the hit lies farther off than the reach (an epsilon above the blend radius): widen
+    *need = reach;
+    return false;
+  }
   struct Frame {
     int inner, stage;
     int i0, im, i1;  // gathered primitives of the left and right child
@@ -835,9 +839,10 @@ __device__ __noinline__ bool resolve_urtree_reach(const DevScene& S, const DevUr
 
 __device__ void resolve_urtree(const DevScene& S, const DevUrTree& t, F3 p, const HookCtx& hc, Resolved* out,
                                bool split_root) {
-  float reach = t.fine.dims[0] > 0 ? ur_list_reach(t.r) : 3.0f * t.r;
+  const bool listed = t.fine.dims[0] > 0;  // one more attempt, within what a cell lists, before 3 r
+  float reach = listed ? ur_list_reach(t.r) : 3.0f * t.r;
   out->ok = false;
-  for (int attempt = 0; attempt < 6; ++attempt) {
+  for (int attempt = listed ? -1 : 0; attempt < 6; ++attempt) {
     float need = 0.0f;
     if (resolve_urtree_reach(S, t, p, hc, reach, out, &need, split_root)) return;
     if (need < 0.0f) return;  // capacity exceeded

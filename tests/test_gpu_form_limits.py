@@ -11,6 +11,7 @@ import pytest
 import forgedthoughts_gb300 as ft
 import oracle
 from forgedthoughts_gb300 import _native, workloads
+from parity import radiance_rmse
 
 pytestmark = pytest.mark.gpu
 
@@ -95,3 +96,25 @@ def test_material_of_a_primitive_nearer_than_the_tree():
     both = (img.mask == 1) & (m == 1)
     assert both.mean() > 0.5 and (mat[both] != 0).all()
     assert (img.material[both] == mat[both]).all()
+
+
+@pytest.mark.parametrize("n", [6, 14])
+def test_resolve_of_hits_farther_off_than_the_blend_radius(n):
+    """An epsilon above the blend radius stops a ray where no primitive is
+    within it: the gather widens instead of giving up (the general resolve of
+    the fallback holds eight open subtrees, a chain of 14 needs more, and its
+    material's hooks were lost)."""
+    from test_frontend import HOOK_MATERIALS
+
+    lines = [f"let s{i} = Sphere {{ radius: 0.35, pos: vec3({-1.6 + 3.2 * i / (n - 1):.4f}, "
+             f"{0.6 + 0.2 * (i % 3):.2f}, {0.1 * (i % 4):.2f}), material: Stripe {{}} }};" for i in range(n)]
+    lines.append(f"let u{n - 1} = s{n - 1};")
+    for i in range(n - 2, -1, -1):  # every left child a sphere: a chain to the right
+        lines.append(f"let u{i} = s{i}.union_round(u{i + 1}, 0.005);")
+    st = ft.parse_and_eval(HOOK_MATERIALS + LIGHTS + "\n".join(lines) + "\nlet scene = u0;\n")
+    opts = ft.RenderOptions(width=120, height=80, max_steps=256, max_dist=30.0, epsilon=0.01, step_scale=0.7)
+    lin, _ = ft.render_trace(st, opts, ft.AccelMode.Bvh, 1, 1)
+    ref, _, _ = oracle.render_trace(st, opts, 1, 1, 1, 32)
+    assert ref.max() > 0.1
+    # the Whitted bar; silhouette pixels whose hit flips count as everywhere
+    assert radiance_rmse(lin, ref) <= 1e-3, radiance_rmse(lin, ref)
