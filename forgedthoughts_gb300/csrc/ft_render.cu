@@ -224,18 +224,26 @@ std::vector<int> choose_exact_leaves(const ftgpu::SceneImage& im) {
 }
 
 
-// Candidate-list entries of all grids of a scene (8 bytes each); a grid past
-// it is dropped, and its points take the tree BVH.
+// Candidate-list entries, and cells, of all grids of a scene (8 bytes each); a
+// grid past either is dropped, and its points take the outer grid or the tree
+// BVH.  A tree's cell lists at least one primitive, so the cells' bound drops no
+// grid that fits the entries'; it holds before the memory is taken, and keeps
+// cell indices far below 2^31.
 constexpr uint64_t kMaxGridEntries = uint64_t(1) << 26;
 
-// Build the cell lists of `jobs` into one cell and one entry array: count,
-// read the totals, drop the grids that would pass the entry cap (their job's
-// `dims` become 0), fill.
+// Build the cell lists of `jobs` into one cell and one entry array: drop the
+// grids past the cell cap (their job's `dims` become 0), count, read the
+// totals, drop those past the entry cap, fill.
 ft_status build_grids(ft_scene* sc, std::vector<GridJob>* jobs) {
   uint64_t n_cells = 0;
   for (GridJob& j : *jobs) {
+    const uint64_t cells = static_cast<uint64_t>(j.dims[0]) * j.dims[1] * j.dims[2];
+    if (n_cells + cells > kMaxGridEntries) {
+      j.dims[0] = 0;
+      continue;
+    }
     j.first = static_cast<int32_t>(n_cells);
-    n_cells += static_cast<uint64_t>(j.dims[0]) * j.dims[1] * j.dims[2];
+    n_cells += cells;
   }
   if (n_cells == 0) return FT_OK;
   auto blocks = [](const GridJob& j) {
@@ -249,7 +257,8 @@ ft_status build_grids(ft_scene* sc, std::vector<GridJob>* jobs) {
   auto* totals = reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(sc->grid_cells) + totals_off);
   FT_CUDA_TRY(cudaMemsetAsync(totals, 0, n_totals * sizeof(unsigned long long)), "cudaMemset(grid)");
   for (size_t k = 0; k < jobs->size(); ++k)
-    grid_cells_kernel<false><<<blocks((*jobs)[k]), 64>>>(sc->dev, (*jobs)[k], sc->grid_cells, nullptr, totals + k);
+    if ((*jobs)[k].dims[0] > 0)
+      grid_cells_kernel<false><<<blocks((*jobs)[k]), 64>>>(sc->dev, (*jobs)[k], sc->grid_cells, nullptr, totals + k);
   FT_CUDA_TRY(cudaGetLastError(), "grid_cells_kernel launch");
   std::vector<unsigned long long> count(n_totals);
   FT_CUDA_TRY(cudaMemcpy(count.data(), totals, n_totals * sizeof(unsigned long long), cudaMemcpyDeviceToHost),

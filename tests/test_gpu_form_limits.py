@@ -118,3 +118,27 @@ def test_resolve_of_hits_farther_off_than_the_blend_radius(n):
     assert ref.max() > 0.1
     # the Whitted bar; silhouette pixels whose hit flips count as everywhere
     assert radiance_rmse(lin, ref) <= 1e-3, radiance_rmse(lin, ref)
+
+
+def test_grids_of_very_many_trees_are_bounded():
+    """Each union_round tree asks for its own cells; past 2^26 of them, or
+    2^26 list entries, further trees keep no grid and take their BVH."""
+    n, lines, roots = 2400, [], []
+    for k in range(n):
+        x, z = (k % 49 - 24) * 0.4, (k // 49 - 24) * 0.4
+        names = [f"s{k}_{i}" for i in range(4)]
+        lines += [f"let {v} = Sphere {{ radius: 0.08, pos: vec3({x + 0.1 * (i % 2):.3f}, {0.1 * (i // 2):.3f}, {z:.3f}) }};"
+                  for i, v in enumerate(names)]
+        ups, root = _tree(names, 0.05, f"u{k}_")
+        lines += ups
+        roots.append(root)
+    st = ft.parse_and_eval(LIGHTS + "\n".join(lines) + "\nlet scene = " + " + ".join(roots) + ";\n")
+    size = ctypes.c_uint64()
+    assert _native.lib().ft_scene_device_bytes(st.gpu().handle, ctypes.byref(size)) == 0
+    assert size.value <= 2 * 8 * 2 ** 26 + 2 ** 26  # cells and entries of 8 bytes; the scene's records
+    opts = ft.RenderOptions(width=64, height=48, max_steps=256, max_dist=40.0, epsilon=1e-4, step_scale=0.7)
+    img = ft.render_depth(st, opts, ft.AccelMode.Bvh, 1)
+    t, m, _, _, _ = oracle.render_depth(st, opts, 1, 1, 32)
+    both = (img.mask == 1) & (m == 1)
+    assert (img.mask == m).mean() >= 0.999 and both.mean() > 0.1
+    assert (np.abs(img.t[both] - t[both]) <= 1e-4).mean() >= 0.999
