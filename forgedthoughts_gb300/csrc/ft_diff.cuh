@@ -509,7 +509,10 @@ __device__ __noinline__ bool scene_backprop(const DevScene& S, F3 p, const DiffT
 // are idle.  Forward (kAdjoint false): depth, mask and silhouette.  Adjoint:
 // the rays that carry an upstream gradient march again and leave a record for
 // views_adjoint_kernel, hits from the front of `records` and misses from its
-// end.  Self-checks as in march_depth_persistent.
+// end.  Self-check: a ray ends after at most max_steps march steps and some 200
+// of refinement; a lane past max_steps + 256 sets a bit in counters[1] and
+// gives up.  There is no time limit: a call is one launch over all its views,
+// however long these take.
 //
 // One thread per ray to the end left a warp waiting for its longest search: a
 // miss takes 40 golden-section steps after its march, and an adjoint ray its
@@ -522,10 +525,9 @@ __global__ void __launch_bounds__(128, 8) views_march_persistent(
     const float* __restrict__ dl_dt, const float* __restrict__ dl_dsil, AdjointRay* __restrict__ records,
     unsigned long long* __restrict__ counters) {
   const unsigned lane = threadIdx.x & 31u;
-  const unsigned long long t_start = __shfl_sync(0xffffffffu, lane == 0 ? ftd::global_ns() : 0ull, 0);
   Ctx<false> cx;
   cx.c = Counters{};
-  uint32_t loop_iters = 0, ray_iters = 0, view = 0;
+  uint32_t ray_iters = 0, view = 0;
   bool queue_done = false;
   ViewRay ray;
   uint64_t item = 0;
@@ -546,14 +548,6 @@ __global__ void __launch_bounds__(128, 8) views_march_persistent(
     }
   };
   for (;;) {
-    if ((++loop_iters & 1023u) == 0u) {
-      unsigned long long now = lane == 0 ? ftd::global_ns() : 0ull;
-      now = __shfl_sync(0xffffffffu, now, 0);
-      if (now - t_start > kMarchWallNs) {
-        if (lane == 0) atomicOr(&counters[1], 1ull << 8);
-        break;
-      }
-    }
     const unsigned idle = __ballot_sync(0xffffffffu, !ray.live());
     if (!queue_done && (__popc(idle) >= kWfRefill || idle == 0xffffffffu)) {
       unsigned long long base = 0;
@@ -593,7 +587,7 @@ __global__ void __launch_bounds__(128, 8) views_march_persistent(
     }
     if (!ray.live()) continue;
     const RayParams& P = views[view];
-    if (++ray_iters > P.max_steps + 256u) {
+    if (++ray_iters > 256u && ray_iters - 256u > P.max_steps) {
       atomicOr(&counters[1], 1ull);
       ray.state = ViewRay::kEmpty;
       finish();

@@ -950,7 +950,7 @@ ft_status march_check(unsigned long long flags) {
     char buf[32];
     std::snprintf(buf, sizeof(buf), "%llx", flags);
     return std::string(buf);
-  }() + "): a ray exceeded max_steps + 64 iterations or a warp ran for over 20 s");
+  }() + "): a ray exceeded the iterations its step limit allows or a warp ran for over 20 s");
 }
 
 // After the batch's work has completed: fail if a Whitted queue overflowed or

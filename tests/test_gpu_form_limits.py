@@ -142,3 +142,36 @@ def test_grids_of_very_many_trees_are_bounded():
     both = (img.mask == 1) & (m == 1)
     assert (img.mask == m).mean() >= 0.999 and both.mean() > 0.1
     assert (np.abs(img.t[both] - t[both]) <= 1e-4).mean() >= 0.999
+
+
+def _hard_fit_scene():
+    return ft.ParamScene(workloads.shape_fit(n=16))
+
+
+def test_views_take_any_step_limit():
+    """A march ends by its own distance limit; a step limit near 2^32 changes
+    nothing."""
+    ps, vs = _hard_fit_scene(), ft.ring_views(2)
+    got = []
+    for steps in (100000, 2 ** 32 - 1):
+        opts = ft.RenderOptions(width=64, height=64, max_steps=steps, max_dist=100.0, epsilon=1e-4, step_scale=0.05)
+        t, mask, sil = ps.render(vs, opts)
+        g = ps.backward(vs, opts, (mask == 1).astype(np.float32), (mask == 0).astype(np.float32))
+        got.append((t, mask, sil, g))
+    assert got[0][1].any()
+    for a, b in zip(got[0][:3], got[1][:3]):
+        assert np.array_equal(a, b)
+    assert np.allclose(got[0][3], got[1][3], rtol=1e-6, atol=1e-6 * np.abs(got[0][3]).max())  # atomics' order
+
+
+def test_views_take_as_long_as_they_need():
+    """A views call is one launch however long it takes (here about 28 s: a
+    thousand shells around one centre, interpreted hooks, short steps)."""
+    lines = ["let twist = fn(p) { return rotate_y(p, p.y * 18.0); };",
+             "let ripple = fn(d, p) { return abs(d + sin(p.y * 120.0) * 0.004) - 0.03; };"]
+    lines += [f"let s{i} = Sphere {{ radius: {1.0 + 0.0001 * i:.4f}, domain: twist, distance_post: ripple }};"
+              for i in range(1300)]
+    ps = ft.ParamScene("\n".join(lines) + "\nlet scene = " + " + ".join(f"s{i}" for i in range(1300)) + ";\n")
+    opts = ft.RenderOptions(width=1024, height=1024, max_steps=4000, max_dist=100.0, epsilon=1e-6, step_scale=0.05)
+    _, mask, _ = ps.render(ft.ring_views(1), opts)
+    assert 0.1 < mask.mean() < 0.4
