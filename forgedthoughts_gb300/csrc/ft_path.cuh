@@ -436,9 +436,10 @@ struct PathPixel {
 };
 constexpr uint32_t kPathStopped = 0x80000000u;
 
-// Samples [first, first + n) of every pixel that has not stopped, one path per
-// thread: neighbouring threads trace neighbouring pixels of one sample.  Their
-// radiance goes to out[(sample - first) * pixels + pixel].
+// Samples [first, first + n) of the pixels [first_pixel, first_pixel +
+// n_pixels) that have not stopped, one path per thread: neighbouring threads
+// trace neighbouring pixels of one sample.  Their radiance goes to
+// out[(sample - first) * n_pixels + pixel - first_pixel].
 //
 // A path is a serial chain of distance evaluations and its length varies from
 // one bounce to max_bounces, so a frame needs many of them in flight: a thread
@@ -447,13 +448,13 @@ constexpr uint32_t kPathStopped = 0x80000000u;
 // 45 with ten blocks per SM instead of the compiler's five).
 __global__ void __launch_bounds__(128, 10) path_sample_kernel(const __grid_constant__ DevScene S,
                                                           const __grid_constant__ RayParams P, uint32_t max_bounces,
-                                                          uint32_t first, uint32_t n,
-                                                          const PathPixel* __restrict__ state, float* __restrict__ out) {
+                                                          uint32_t first, uint32_t n, uint64_t first_pixel,
+                                                          uint64_t n_pixels, const PathPixel* __restrict__ state,
+                                                          float* __restrict__ out) {
   const uint64_t g = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const uint64_t n_pixels = static_cast<uint64_t>(P.width) * P.height;
   if (g >= n_pixels * n) return;
-  const uint64_t i = g % n_pixels;
-  if (state[i].count & kPathStopped) return;
+  if (state[g % n_pixels].count & kPathStopped) return;
+  const uint64_t i = first_pixel + g % n_pixels;
   Ctx<false> cx;
   cx.c = Counters{};
   const uint32_t s = first + static_cast<uint32_t>(g / n_pixels);
@@ -474,12 +475,14 @@ __global__ void __launch_bounds__(128, 10) path_sample_kernel(const __grid_const
 }
 
 // The pass's samples into each pixel in order, with the progressive
-// renderer's adaptive stopping; samples behind the stop are dropped.  With
-// `last` the outputs: the average (linear), its spectrum_to_rgb8 (R:5221-5227)
-// and the samples taken.
+// renderer's adaptive stopping; samples behind the stop are dropped.  `active`
+// (nullable) counts the pixels that have not stopped.  With `last` the outputs
+// (arrays of these pixels): the average (linear), its spectrum_to_rgb8
+// (R:5221-5227) and the samples taken.
 __global__ void __launch_bounds__(128) path_accumulate_kernel(uint64_t n_pixels, PathSettingsD ps, uint32_t n,
                                                               const float* __restrict__ in,
-                                                              PathPixel* __restrict__ state, int last,
+                                                              PathPixel* __restrict__ state,
+                                                              unsigned int* __restrict__ active, int last,
                                                               float* __restrict__ rgb_out,
                                                               uint8_t* __restrict__ rgb8_out,
                                                               uint32_t* __restrict__ count_out) {
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(128) path_accumulate_kernel(uint64_t n_pixels,
     st.m2 = m2;
     st.count = count | (stopped ? kPathStopped : 0u);
     state[i] = st;
+    if (active && !stopped) atomicAdd(active, 1u);
     return;
   }
   const F3 avg = count ? sum * (1.0f / static_cast<float>(count)) : f3(0.0f, 0.0f, 0.0f);

@@ -977,8 +977,11 @@ ft_status check_tuning(const ft_batch_tuning& t) {
 
 
 
-// Path samples of one pass (12 bytes each).
+// Path samples of one pass (12 bytes each), pixels of one band (24 bytes of
+// state each), and passes between two looks at the pixels still active.
 constexpr uint64_t kPathSamples = uint64_t(1) << 24;
+constexpr uint64_t kPathPixels = uint64_t(1) << 22;
+constexpr uint32_t kPathCheck = 8;
 
 // Whitted trace of one frame as a wavefront: per bounce level one march, one
 // shade and one shadow kernel over queues (ft_wavefront.cuh).  Radiance per
@@ -1355,29 +1358,53 @@ ft_status ft_render_pathtrace(ft_scene* sc, const ft_render_options* options, ft
   float* rgbf = rgb_out ? (dev_ptrs ? rgb_out : sc->d_rgbf) : nullptr;
   uint8_t* rgb8 = rgb8_out ? (dev_ptrs ? rgb8_out : sc->d_rgb) : nullptr;
   uint32_t* cnt = samples_out ? (dev_ptrs ? samples_out : sc->d_mat) : nullptr;
-  // Passes of samples: the first takes the min_spp that every pixel needs,
-  // later ones at most as many (samples behind a pixel's stop are wasted),
-  // bounded by the sample buffer.
-  const uint64_t cap = std::max<uint64_t>(1, kPathSamples / pixels);
+  // Bands of pixels, and per band passes of samples: the first takes the
+  // min_spp that every pixel needs, later ones at most as many (samples behind
+  // a pixel's stop are wasted), bounded by the sample buffer.
+  const uint64_t band = std::min<uint64_t>(pixels, kPathPixels);
+  const uint64_t cap = std::max<uint64_t>(1, kPathSamples / band);
   const uint32_t most = static_cast<uint32_t>(
-      std::min<uint64_t>(cap, ps.noise_threshold > 0.0f ? std::max(ps.min_spp, 4u) : ps.spp));
-  const uint64_t floats = 3 * pixels * std::min(most, ps.spp) + pixels * (sizeof(PathPixel) / sizeof(float));
+      std::min<uint64_t>({cap, ps.noise_threshold > 0.0f ? std::max(ps.min_spp, 4u) : ps.spp, ps.spp}));
+  constexpr uint64_t kStateFloats = sizeof(PathPixel) / sizeof(float);
+  const uint64_t floats = band * kStateFloats + 3 * band * most + 1;
   if (ft_status s = grow(&sc->path_buf, &sc->path_cap, floats, "cudaMalloc(path samples)")) return s;
   auto* state = reinterpret_cast<PathPixel*>(sc->path_buf);
-  float* samples = sc->path_buf + pixels * (sizeof(PathPixel) / sizeof(float));
-  FT_CUDA_TRY(cudaMemsetAsync(state, 0, pixels * sizeof(PathPixel), st), "memset");
+  float* samples = sc->path_buf + band * kStateFloats;
+  auto* active = reinterpret_cast<unsigned int*>(samples + 3 * band * most);
   sc->last_launches = 0;
-  for (uint32_t first = 0; first < ps.spp;) {
-    const uint32_t n = std::min(ps.spp - first, most);
-    const uint64_t blocks = (pixels * n + 127) / 128;
-    path_sample_kernel<<<static_cast<unsigned>(blocks), 128, 0, st>>>(sc->dev, P, ps.max_bounces, first, n, state,
-                                                                      samples);
-    FT_CUDA_TRY(cudaGetLastError(), "path_sample_kernel launch");
-    first += n;
-    path_accumulate_kernel<<<static_cast<unsigned>((pixels + 127) / 128), 128, 0, st>>>(
-        pixels, ps, n, samples, state, first >= ps.spp ? 1 : 0, rgbf, rgb8, cnt);
-    FT_CUDA_TRY(cudaGetLastError(), "path_accumulate_kernel launch");
-    sc->last_launches += 2;
+  for (uint64_t at = 0; at < pixels; at += band) {
+    const uint64_t n_px = std::min(band, pixels - at);
+    const unsigned px_blocks = static_cast<unsigned>((n_px + 127) / 128);
+    auto accumulate = [&](uint32_t n, bool count, bool last) -> ft_status {
+      path_accumulate_kernel<<<px_blocks, 128, 0, st>>>(n_px, ps, n, samples, state, count ? active : nullptr,
+                                                        last ? 1 : 0, rgbf ? rgbf + 3 * at : nullptr,
+                                                        rgb8 ? rgb8 + 3 * at : nullptr, cnt ? cnt + at : nullptr);
+      FT_CUDA_TRY(cudaGetLastError(), "path_accumulate_kernel launch");
+      sc->last_launches += 1;
+      return FT_OK;
+    };
+    FT_CUDA_TRY(cudaMemsetAsync(state, 0, n_px * sizeof(PathPixel), st), "memset");
+    uint32_t pass = 0;
+    for (uint32_t first = 0; first < ps.spp;) {
+      const uint32_t n = std::min(ps.spp - first, most);
+      // every kPathCheck passes the pixels still active are counted and read
+      // back: the sample limit may be far above what the threshold takes
+      const bool check = ++pass % kPathCheck == 0 && first + n < ps.spp && ps.noise_threshold > 0.0f;
+      if (check) FT_CUDA_TRY(cudaMemsetAsync(active, 0, sizeof(*active), st), "memset");
+      path_sample_kernel<<<static_cast<unsigned>((n_px * n + 127) / 128), 128, 0, st>>>(
+          sc->dev, P, ps.max_bounces, first, n, at, n_px, state, samples);
+      FT_CUDA_TRY(cudaGetLastError(), "path_sample_kernel launch");
+      sc->last_launches += 1;
+      first += n;
+      if (ft_status s = accumulate(n, check, first >= ps.spp)) return s;
+      if (!check) continue;
+      unsigned int left = 0;
+      FT_CUDA_TRY(cudaMemcpyAsync(&left, active, sizeof(left), cudaMemcpyDeviceToHost, st), "copy active pixels");
+      FT_CUDA_TRY(cudaStreamSynchronize(st), "path trace");
+      if (left > 0) continue;
+      if (ft_status s = accumulate(0, false, true)) return s;
+      break;
+    }
   }
   if (!dev_ptrs) {
     if (rgb_out) FT_CUDA_TRY(cudaMemcpyAsync(rgb_out, rgbf, pixels * 3 * sizeof(float), cudaMemcpyDeviceToHost, st),

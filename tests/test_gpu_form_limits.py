@@ -175,3 +175,53 @@ def test_views_take_as_long_as_they_need():
     opts = ft.RenderOptions(width=1024, height=1024, max_steps=4000, max_dist=100.0, epsilon=1e-6, step_scale=0.05)
     _, mask, _ = ps.render(ft.ring_views(1), opts)
     assert 0.1 < mask.mean() < 0.4
+
+
+def _path(st, opts, spp, min_spp, threshold):
+    return ft.render_pathtrace(st, opts, ft.AccelMode.Bvh,
+                               ft.PathtraceSettings(spp=spp, min_spp=min_spp, noise_threshold=threshold))
+
+
+def test_path_ends_with_its_last_pixel():
+    """Once every pixel has reached its noise threshold no further pass is
+    launched, whatever the sample limit, and the result is the one at a limit
+    that the last pixel just reaches."""
+    w = workloads.union_round_field(n=16, seed=2, width=24, height=16, aa=1)
+    st = ft.parse_and_eval(w.source)
+    many = _path(st, w.options, 65536, 2, 0.5)
+    launches = ctypes.c_uint32()
+    assert _native.lib().ft_scene_last_launches(st.gpu().handle, ctypes.byref(launches)) == 0
+    most = int(many[2].max())
+    assert most < 1024
+    assert launches.value <= 2 * (most // 4 + 1) + 64
+    few = _path(st, w.options, most, 2, 0.5)
+    for a, b in zip(many, few):
+        assert np.array_equal(a, b)
+
+
+def test_path_buffers_do_not_grow_with_the_frame():
+    """A large frame is traced in bands: beyond the frame's own buffers (which
+    the depth preview has too) at most 2^24 samples of 12 bytes and the state
+    of a band.  Rows of every band against the f32 oracle, at the bars of the
+    path tracer's other comparisons."""
+    torch = pytest.importorskip("torch")
+    st = ft.parse_and_eval(LIGHTS + "let scene = Sphere { radius: 0.9, pos: vec3(0, 0.6, 0) };")
+    opts = ft.RenderOptions(width=6144, height=4096, max_steps=64, max_dist=20.0, epsilon=1e-3, step_scale=0.9)
+    h, o = st.gpu().handle, opts.to_c()
+    lib = _native.lib()
+    assert lib.ft_render_depth(h, ctypes.byref(o), 1, 1, None, None, None, None, None, 0, None) == 0
+    count = torch.zeros(opts.height, opts.width, dtype=torch.int32, device="cuda")
+    rgb = torch.zeros(opts.height, opts.width, 3, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    settings = _native.PathtraceSettingsC(2, 1, 1, 0.0)
+    assert lib.ft_render_pathtrace(h, ctypes.byref(o), 1, ctypes.byref(settings), ctypes.c_void_p(rgb.data_ptr()),
+                                   None, ctypes.c_void_p(count.data_ptr()), _native.FT_FLAG_DEVICE_POINTERS, None) == 0
+    assert free - torch.cuda.mem_get_info()[0] <= 12 * 2 ** 24 + 2 ** 27
+    assert (count == 2).all()
+    ref, _, _, _ = oracle.render_path(st, opts, 1, spp=2, max_bounces=1, min_spp=1, noise_threshold=0.0,
+                                      rows=(300, 4096, 500))
+    rows = np.arange(300, 4096, 500)
+    got, ref = rgb.cpu().numpy()[rows].astype(np.float64), ref[rows]
+    assert ref.max() > 0.1
+    assert (np.abs(got - ref).max(axis=-1) <= 1e-3).mean() >= 0.99 and radiance_rmse(got, ref) <= 2e-2
