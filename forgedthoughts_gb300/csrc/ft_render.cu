@@ -276,7 +276,6 @@ ft_status build_grids(ft_scene* sc, std::vector<GridJob>* jobs) {
     if (j.dims[0] > 0)
       grid_cells_kernel<true><<<blocks(j), 64>>>(sc->dev, j, sc->grid_cells, sc->grid_entries, totals + jobs->size());
   FT_CUDA_TRY(cudaGetLastError(), "grid_cells_kernel launch");
-  FT_CUDA_TRY(cudaStreamSynchronize(nullptr), "grid build");  // renders run on any stream
   return FT_OK;
 }
 
@@ -574,6 +573,10 @@ ft_status upload_scene(ft_scene* sc) {
   FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, true, false>, 128, 0),
               "occupancy");
   sc->persistent_blocks_bricks = std::max(1, sms * std::max(per_sm, 1));
+  // Renders run on any stream, also on ones that do not wait for this one: the
+  // copies (a pageable copy may still be on its way when the call returns) and
+  // the grids are complete from here on.
+  FT_CUDA_TRY(cudaStreamSynchronize(nullptr), "scene upload");
   return FT_OK;
 }
 

@@ -225,3 +225,21 @@ def test_path_buffers_do_not_grow_with_the_frame():
     got, ref = rgb.cpu().numpy()[rows].astype(np.float64), ref[rows]
     assert ref.max() > 0.1
     assert (np.abs(got - ref).max(axis=-1) <= 1e-3).mean() >= 0.99 and radiance_rmse(got, ref) <= 2e-2
+
+
+@pytest.mark.parametrize("n", [4, 64])
+def test_a_new_scene_is_complete_for_every_stream(n):
+    """A scene rendered straight after its creation on a stream that does not
+    wait for the default stream: the frame it gives later."""
+    torch = pytest.importorskip("torch")
+    w = workloads.union_round_field(n=n, seed=4, width=320, height=180, aa=1)
+    stream, o = torch.cuda.Stream(), w.options.to_c()
+    st = ft.parse_and_eval(w.source)
+    t = [torch.zeros(180 * 320, dtype=torch.float32, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    for x in t:
+        assert _native.lib().ft_render_depth(st.gpu().handle, ctypes.byref(o), 1, 1, ctypes.c_void_p(x.data_ptr()), None,
+                                             None, None, None, _native.FT_FLAG_DEVICE_POINTERS,
+                                             ctypes.c_void_p(stream.cuda_stream)) == 0
+        torch.cuda.synchronize()
+    assert (t[0] > 0).any() and torch.equal(t[0], t[1])
