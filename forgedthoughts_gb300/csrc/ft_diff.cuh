@@ -359,7 +359,7 @@ __device__ __noinline__ bool urtree_backprop(const DevScene& S, int ti, F3 p, co
       if (__uint_as_float(e.x) >= ftd::rmax(t.r, best.d)) break;
       const int i = static_cast<int>(e.y & ~ftd::kRareFlag);
       const float d = ftd::prim_distance(S.nodes[S.ur_prims[i]], p);
-      if (d < best.d) best = Info{d, ~i};
+      if (d < best.d || (d == best.d && i > ~best.ref)) best = Info{d, ~i};  // (equal: the later one's, as in the fold)
       if (d < t.r) {
         if (nn < kNear) idx[nn] = i;
         ++nn;
@@ -368,6 +368,7 @@ __device__ __noinline__ bool urtree_backprop(const DevScene& S, int ti, F3 p, co
   } else {
     bool tie;
     best = far_nearest<false>(S, t, p, best, &tie, cx);
+    if (tie) return urtree_backprop_full(S, ti, p, T, g);
   }
   if (nn > kNear || best.ref == ftd::kNoRef) return urtree_backprop_full(S, ti, p, T, g);
   if (nn == 0) {

@@ -495,7 +495,7 @@ __device__ __forceinline__ Info ur_value(const DevScene& S, const DevUrTree& t, 
 
 // Nearest primitive below best.d from a point outside the candidate grids,
 // where every primitive is outside its box: the nodes in depth-first order, a
-// subtree skipped when its box is not nearer than the best so far.  Out of
+// subtree skipped when its box is farther than the best so far.  Out of
 // line: it is rare beside the grids' cell walks, whose code stays in the march
 // loops.  A node is two 16-byte loads and there is no stack: the leaf-BVH walk
 // it replaces for these points spent over a thousand cycles on a node (14
@@ -511,7 +511,7 @@ __device__ __noinline__ Info far_nearest(const DevScene& S, const DevUrTree& t, 
     const float4 b = __ldg(S.far_nodes + 2 * static_cast<size_t>(k) + 1);
     const float mn[3] = {a.x, a.y, a.z}, mx[3] = {b.x, b.y, b.z};
     cx.box();
-    if (ftd::aabb_lb2(p, mn, mx) >= best.d * best.d) {
+    if (ftd::aabb_lb2(p, mn, mx) > 1.000001f * best.d * best.d) {  // (not an equally near one, whatever the rounding)
       k = __float_as_int(a.w);
       continue;
     }

@@ -243,3 +243,25 @@ def test_a_new_scene_is_complete_for_every_stream(n):
                                              ctypes.c_void_p(stream.cuda_stream)) == 0
         torch.cuda.synchronize()
     assert (t[0] > 0).any() and torch.equal(t[0], t[1])
+
+
+@pytest.mark.parametrize("extra", [0, 1, 5])
+def test_adjoint_of_equally_near_primitives(extra):
+    """Where two primitives are equally far and none within the blend radius,
+    the whole derivative is the later one's (the folds take `a < b ? a : b`),
+    as in the FP64 adjoint: mirrored spheres seen along their plane."""
+    lines = [f"let p{i} = Sphere {{ radius: 0.3, pos: vec3({x}, {y}, 0.0) }};"
+             for i, (x, y) in enumerate([(-1.0, 0.0), (1.0, 0.0), (-1.0, 1.5), (1.0, 1.5)])]
+    lines += [f"let p{4 + i} = Sphere {{ radius: 0.2, pos: vec3({6 + i}, 4, 0.5) }};" for i in range(extra)]
+    ups, root = _tree([f"p{i}" for i in range(4 + extra)], 0.1)
+    ps = ft.ParamScene("\n".join(lines + ups) + f"\nlet scene = {root};\n")
+    vs = [((0.0, 0.0, -5.0), (0.0, 0.0, 0.0), 40.0)]
+    opts = workloads.shape_fit_options(33)  # odd: the middle column looks along x = 0
+    _, mask, sil = ps.render(vs, opts, 0.2)
+    ws = np.zeros(mask.shape, np.float32)
+    ws[0, 14:19, 16] = 1.0
+    assert (mask[ws > 0] == 0).all() and (sil[ws > 0] > 1e-3).all()
+    g = ps.backward(vs, opts, None, ws, 0.2)
+    ref = oracle.render_backward(ps.state, vs, opts, ps.layout, None, ws, 0.2, 64)
+    # FP32 positions of the minima: the bound of the other gradient comparisons
+    assert np.abs(g - ref).max() <= 2e-2 * np.abs(ref).max(), (g, ref)
