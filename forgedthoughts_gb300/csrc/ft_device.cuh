@@ -170,7 +170,8 @@ FT_DEV float prim_distance(const DevNode& n, F3 p) { return prim_local(n.kind, n
 //   { centre, cos }, { h, rd }, { sin, shell, node, leaf | rare flag }
 // with the sin / cos of DevNode, h the box's half size less its rounding rd
 // (0 and the radius for a sphere, whose distance is that of a box of no size
-// rounded by the radius) and shell = +inf where there is none.  One branch-free
+// rounded by the radius; its h.x is -0, which no box's is) and shell = +inf
+// where there is none.  One branch-free
 // formula in 48 bytes serves every lane; each term is the one prim_local
 // computes (the sphere's |q| - 0, the unturned box's 1 q.x + 0 q.z and the
 // absent shell's max(d, -inf) are exact).  The multiply-adds are written out:
@@ -178,9 +179,10 @@ FT_DEV float prim_distance(const DevNode& n, F3 p) { return prim_local(n.kind, n
 // it, so that the depth march and the wavefront march take the same steps.
 // Other kinds set the rare flag and go through their node.
 //
-// kSphereYX: a sphere's squares are summed y first, as sphere_local does: a
-// hard union's spheres have always rounded that way, a union_round tree's
-// x first, and an ulp of a distance moves a silhouette pixel.
+// kSphereYX: a sphere's squares are summed y first, as sphere_local does, a
+// box's (also one rounded to its whole size) x first, as box_local does: a
+// hard union's have always rounded that way, a union_round tree's x first, and
+// an ulp of a distance moves a silhouette pixel.
 constexpr uint32_t kRareFlag = 0x80000000u;
 template <bool kSphereYX>
 FT_DEV float compact_distance(float4 a, float4 b, float sn, float sh, F3 p) {
@@ -188,7 +190,7 @@ FT_DEV float compact_distance(float4 a, float4 b, float sn, float sh, F3 p) {
   const float qx = fabsf(fmaf(a.w, t.x, sn * t.z)) - b.x, qy = fabsf(t.y) - b.y,
               qz = fabsf(fmaf(a.w, t.z, -sn * t.x)) - b.z;
   const float ox = rmax(qx, 0.0f), oy = rmax(qy, 0.0f), oz = rmax(qz, 0.0f);
-  const bool yx = kSphereYX && b.x == 0.0f;
+  const bool yx = kSphereYX && __float_as_uint(b.x) == 0x80000000u;
   const float u = yx ? oy : ox, v = yx ? ox : oy;
   const float outside = sqrtf(fmaf(oz, oz, fmaf(u, u, v * v)));
   const float inside = rmin(rmax(rmax(qx, qy), qz), 0.0f);

@@ -965,6 +965,7 @@ CompactPrim compact_prim(const SceneImage& img, int node, uint32_t leaf) {
   c.shell = shell > 0.0f ? shell : std::numeric_limits<float>::infinity();
   c.rd = n.kind == FT_NODE_SPHERE ? n.f[0] : n.f[3];
   for (int a = 0; a < 3; ++a) c.h[a] = n.kind == FT_NODE_SPHERE ? 0.0f : std::max(n.f[a] - n.f[3], 0.0f);
+  if (n.kind == FT_NODE_SPHERE) c.h[0] = -0.0f;  // marks a sphere
   return c;
 }
 

@@ -40,7 +40,7 @@ struct HostBvhNode {  // leaf BVH in the reference's build order (R:693-732)
 
 struct CompactPrim {  // the device's three 16-byte words (compact_distance)
   float c[3], cos;
-  float h[3], rd;
+  float h[3], rd;  // (h[0] is -0 for a sphere)
   float sin, shell;
   int32_t node;
   uint32_t leaf;  // leaf index, high bit: not a compact kind, evaluated through its node

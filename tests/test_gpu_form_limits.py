@@ -265,3 +265,19 @@ def test_adjoint_of_equally_near_primitives(extra):
     ref = oracle.render_backward(ps.state, vs, opts, ps.layout, None, ws, 0.2, 64)
     # FP32 positions of the minima: the bound of the other gradient comparisons
     assert np.abs(g - ref).max() <= 2e-2 * np.abs(ref).max(), (g, ref)
+
+
+def test_round_boxes_and_spheres_keep_their_own_summation():
+    """A box rounded to its half size has an empty core like a sphere's, but
+    its squares are summed in a box's order: among hard-unioned primitives it
+    has the distance, to the bit, that it has beside a boolean, where every
+    primitive is evaluated from its node."""
+    lines = ["let a = Box { size: vec3(0.8, 0.8, 0.8), round: 0.4, pos: vec3(-0.7, 0.5, 0.1) };",
+             "let b = Box { size: vec3(0.6, 1.2, 0.7), round: 0.3, pos: vec3(0.7, 0.6, -0.2), rot: vec3(0, 25, 0) };",
+             "let c = Sphere { radius: 0.35, pos: vec3(0.1, 0.4, 0.9) };",
+             "let d = Box { size: vec3(20, 0.2, 20), pos: vec3(0, 60, 0) };",
+             "let e = Box { size: vec3(20, 0.2, 20), pos: vec3(0, 61, 0) };"]
+    pts = _points(40000, 2.5)
+    fast = ft.parse_and_eval("\n".join(lines) + "\nlet scene = a + b + c + d;\n")
+    general = ft.parse_and_eval("\n".join(lines) + "\nlet scene = a + b + c + (d - e);\n")
+    assert np.array_equal(_distances(fast, pts), _distances(general, pts))
