@@ -780,7 +780,11 @@ struct ft_batch {
   // they never touch them under a launch still running on another stream.
   cudaEvent_t done = nullptr;
   cudaGraphExec_t exec = nullptr;
-  ft_batch_tuning tuning{8, 8, 24, 0.0f};
+  // The default is one of the autotuner's candidates, so that tuning cannot
+  // leave a batch slower than it was.  (32 uneven scenes: 23.2 ms at 24 idle
+  // lanes, 23.4 at 16, 23.8 at 8; one 1280x720 frame of the 512-primitive field:
+  // 1.88, 1.98, 2.06.)
+  ft_batch_tuning tuning{8, 8, 16, 0.0f};
   std::mutex mu;
   // Wavefront queues of the trace items (sized per tuning: tiles pad the
   // work items), their counters (job counts x2, shadow count, overflow
