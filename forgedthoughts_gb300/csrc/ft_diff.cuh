@@ -350,6 +350,7 @@ __device__ __noinline__ bool urtree_backprop(const DevScene& S, int ti, F3 p, co
   int idx[kNear];
   int nn = 0;
   Info best{kInf, ftd::kNoRef};
+  bool tie = false;
   Ctx<false> cx;
   cx.c = Counters{};
   if (grid_cell(t.fine, p, &cell) || grid_cell(t.outer, p, &cell)) {
@@ -359,18 +360,17 @@ __device__ __noinline__ bool urtree_backprop(const DevScene& S, int ti, F3 p, co
       if (__uint_as_float(e.x) >= ftd::rmax(t.r, best.d)) break;
       const int i = static_cast<int>(e.y & ~ftd::kRareFlag);
       const float d = ftd::prim_distance(S.nodes[S.ur_prims[i]], p);
-      if (d < best.d || (d == best.d && i > ~best.ref)) best = Info{d, ~i};  // (equal: the later one's, as in the fold)
+      const int ref = d < best.d ? ~i : min(~i, best.ref);
+      if (d <= best.d) best = Info{d, ref};  // (equal: the later one's, as in the fold)
       if (d < t.r) {
         if (nn < kNear) idx[nn] = i;
         ++nn;
       }
     }
   } else {
-    bool tie;
     best = far_nearest<false>(S, t, p, best, &tie, cx);
-    if (tie) return urtree_backprop_full(S, ti, p, T, g);
   }
-  if (nn > kNear || best.ref == ftd::kNoRef) return urtree_backprop_full(S, ti, p, T, g);
+  if (nn > kNear || best.ref == ftd::kNoRef || tie) return urtree_backprop_full(S, ti, p, T, g);
   if (nn == 0) {
     const int node = S.ur_prims[~best.ref];
     prim_backprop(S.nodes[node], node, p, 1.0f, g);
