@@ -281,3 +281,56 @@ def test_round_boxes_and_spheres_keep_their_own_summation():
     fast = ft.parse_and_eval("\n".join(lines) + "\nlet scene = a + b + c + d;\n")
     general = ft.parse_and_eval("\n".join(lines) + "\nlet scene = a + b + c + (d - e);\n")
     assert np.array_equal(_distances(fast, pts), _distances(general, pts))
+
+
+def test_the_adjoint_marches_the_forward_rays():
+    """The adjoint re-marches each ray, so it must find what the forward pass
+    found: a silhouette gradient on the forward pass's hits alone, or a depth
+    gradient on its misses alone, reaches no parameter."""
+    ps, vs = ft.ParamScene(workloads.shape_fit(n=64)), ft.ring_views(24)
+    opts = workloads.shape_fit_options(512)
+    _, mask, _ = ps.render(vs, opts)
+    assert 0.02 < mask.mean() < 0.98
+    assert not ps.backward(vs, opts, None, (mask == 1).astype(np.float32)).any()
+    assert not ps.backward(vs, opts, (mask == 0).astype(np.float32), None).any()
+
+
+def test_crowded_hard_union():
+    """More primitives in one block of cells than a block keeps (2048), and
+    lists long enough for the heap sort: spheres around nearly one centre."""
+    rng = np.random.default_rng(3)
+    lines = [f"let s{i} = Sphere {{ radius: {0.5 + 4e-5 * i:.5f}, pos: vec3({x:.4f}, {y:.4f}, {z:.4f}) }};"
+             for i, (x, y, z) in enumerate(rng.uniform(-0.05, 0.05, size=(2500, 3)))]
+    st = ft.parse_and_eval("\n".join(lines) + "\nlet scene = " + " + ".join(f"s{i}" for i in range(2500)) + ";\n")
+    pts = np.concatenate([_points(6000, r) for r in (0.8, 1.5, 8.0)])
+    ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
+    err = np.abs(_distances(st, pts) - ref)
+    assert (err <= 1e-5 * np.maximum(1.0, np.abs(ref))).all(), (float(err.max()), pts[err.argmax()])
+
+
+def test_tree_whose_grids_are_dropped():
+    """1200 nearly concentric spheres pass the cap of 2^26 list entries: the
+    tree keeps no grid and is evaluated through its BVH or its whole fold."""
+    from test_scene_build import _overlapping_spheres
+
+    st = ft.parse_and_eval(_overlapping_spheres(1200))
+    size = ctypes.c_uint64()
+    assert _native.lib().ft_scene_device_bytes(st.gpu().handle, ctypes.byref(size)) == 0
+    assert size.value < 8 * 2 ** 26
+    pts = np.concatenate([_points(700, r) + np.float32([0, 1, 0]) for r in (0.8, 1.5, 8.0)])
+    ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
+    err = np.abs(_distances(st, pts) - ref)
+    assert (err <= 1e-5 * np.maximum(1.0, np.abs(ref))).all(), (float(err.max()), pts[err.argmax()])
+
+
+def test_adjoint_in_chunks_of_rays():
+    """More rays than one pass of the adjoint takes (2^22): the sum of the
+    views' own gradients, up to the order of the FP32-weighted FP64 sums."""
+    ps, vs = ft.ParamScene(workloads.shape_fit(n=16)), ft.ring_views(5)
+    opts = workloads.shape_fit_options(1024)
+    rng = np.random.default_rng(2)
+    w = [rng.normal(size=(5, 1024, 1024)).astype(np.float32) for _ in range(2)]
+    whole = ps.backward(vs, opts, w[0], w[1])
+    parts = sum(ps.backward(vs[k:k + 1], opts, w[0][k:k + 1], w[1][k:k + 1]) for k in range(5))
+    assert np.abs(whole).max() > 0
+    assert np.abs(whole - parts).max() <= 1e-9 * np.abs(parts).max()
