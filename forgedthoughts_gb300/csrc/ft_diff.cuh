@@ -519,7 +519,7 @@ __device__ __noinline__ bool scene_backprop(const DevScene& S, F3 p, const DiffT
 // miss takes 40 golden-section steps after its march, and an adjoint ray its
 // gradient.  Eight blocks per SM (64 registers): 11.4 ms for the step above
 // against 12.4 with five.
-template <bool kAdjoint>
+template <bool kAdjoint, int kForm>
 __global__ void __launch_bounds__(128, 8) views_march_persistent(
     const __grid_constant__ DevScene S, const RayParams* __restrict__ views, uint64_t items_per_view, uint64_t first,
     uint64_t n_work, float tau, float* __restrict__ t_out, uint8_t* __restrict__ mask_out, float* __restrict__ sil_out,
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(128, 8) views_march_persistent(
       finish();
       continue;
     }
-    ray.next(P, max_t, scene_distance_inl(S, o + d * ray.t, cx).d);
+    ray.next(P, max_t, scene_distance_inl<kForm>(S, o + d * ray.t, cx).d);
     if (!ray.live()) finish();
   }
 }

@@ -72,14 +72,18 @@ struct DevUrInner {
 //   kFastPair   two primitives (entry and boxes 0, 1: the BVH root's children);
 //   kFastUnion  primitives only: the first n_always compact records at every
 //               point, the others through the candidate grids and far walk of
-//               `tree`, box 1 around them.
-enum FastKind : int32_t { kFastNone = 0, kFastTree = 1, kFastPair = 2, kFastUnion = 3 };
+//               `tree`, box 1 around them;
+//   kFastLeaves one or two leaves of any other kinds (leaf and boxes 0, 1; one
+//               leaf is leaf[1], with leaf[0] -1), entry[k] where leaf k is a
+//               primitive.
+enum FastKind : int32_t { kFastLeaves = -1, kFastNone = 0, kFastTree = 1, kFastPair = 2, kFastUnion = 3 };
 struct alignas(16) DevFast {
   int32_t kind;
   int32_t n_always;
   int32_t tree_lhs;   // kFastTree: the tree is the BVH root's left child
   int32_t all;        // kFastUnion: every primitive is in the first n_always
   uint32_t entry[2];  // compact entries, kNoPrim for none
+  int32_t leaf[2];    // kFastLeaves
   float4 rec[3];      // the compact record of entry[0], or of the first always-evaluated primitive
   float bmin[2][3], bmax[2][3];
   DevUrTree tree;
@@ -732,14 +736,10 @@ __device__ __noinline__ Info eval_hooked_record(const DevScene& S, int record, F
   return Info{d, __float_as_int(c.z)};
 }
 
+// A leaf other than a primitive.
 template <bool kStats>
-__device__ __forceinline__ Info eval_leaf(const DevScene& S, int leaf, F3 p, float cutoff, Ctx<kStats>& cx) {
-  const int4 info = __ldg(S.leaf_info + leaf);  // kind, node, first, count
-  if (info.x == ftgpu::kLeafPrim) {
-    const DevNode& n = S.nodes[info.y];
-    cx.prim();
-    return Info{ftd::prim_distance(n, p), info.y};
-  }
+__device__ __forceinline__ Info eval_composite(const DevScene& S, int leaf, int4 info, F3 p, float cutoff,
+                                               Ctx<kStats>& cx) {
   if (info.x == ftgpu::kLeafHooked)
     return info.z >= 0 ? eval_hooked_record(S, info.z, p, cx) : eval_hooked(S, info.y, p, cx);
   if (info.x == ftgpu::kLeafUrTree) return eval_urtree_leaf(S, S.urtrees[info.z], p, cutoff, cx);
@@ -757,6 +757,17 @@ __device__ __forceinline__ Info eval_leaf(const DevScene& S, int leaf, F3 p, flo
   return eval_generic(S, info.z, info.w, p, cx);
 }
 
+template <bool kStats>
+__device__ __forceinline__ Info eval_leaf(const DevScene& S, int leaf, F3 p, float cutoff, Ctx<kStats>& cx) {
+  const int4 info = __ldg(S.leaf_info + leaf);  // kind, node, first, count
+  if (info.x == ftgpu::kLeafPrim) {
+    const DevNode& n = S.nodes[info.y];
+    cx.prim();
+    return Info{ftd::prim_distance(n, p), info.y};
+  }
+  return eval_composite(S, leaf, info, p, cutoff, cx);
+}
+
 // Accelerator::distance_info over the leaf BVH (bvh_distance_info,
 // R:743-786): nearest-first, a node is skipped when its box bound exceeds the
 // best distance so far, a later leaf replaces the result only when strictly
@@ -770,46 +781,6 @@ __device__ __noinline__ Info scene_distance_bvh(const DevScene& S, F3 p, Ctx<kSt
     if (in.d < cur.d) cur = in;
   }
   return cur;
-}
-
-// The nearer leaf, then the other when its box bound is not above the
-// distance found (the strictly-closer replace of bvh_distance_info).  One
-// evaluation site for both leaves: the leaf evaluator (with the whole
-// union_round path) is inlined once, which keeps the march loops' code within
-// the instruction cache.
-template <bool kStats>
-__device__ __forceinline__ Info scene_distance_leaves(const DevScene& S, F3 p, int leaf, int second, float second_lb,
-                                                      Ctx<kStats>& cx) {
-  Info cur{kInf, ftd::kNoRef};
-#pragma unroll 1
-  for (int k = 0; k < 2; ++k) {
-    const Info in = eval_leaf(S, leaf, p, k == 0 ? kInf : cur.d, cx);
-    if (k == 0 || in.d < cur.d) cur = in;
-    if (second < 0 || !(second_lb <= cur.d)) break;
-    leaf = second;
-  }
-  return cur;
-}
-
-// Same traversal, with the one- and two-leaf BVHs (a single object, or a
-// ground plus one composite object) walked without a stack.
-template <bool kStats>
-__device__ __noinline__ Info scene_distance_general(const DevScene& S, F3 p, Ctx<kStats>& cx) {
-  const DevBvhNode& root = S.bvh[S.bvh_root];
-  int leaf = root.leaf, second = -1;
-  float second_lb = kInf;
-  if (leaf < 0) {
-    const DevBvhNode& L = S.bvh[root.lhs];
-    const DevBvhNode& R = S.bvh[root.rhs];
-    if (L.leaf < 0 || R.leaf < 0) return scene_distance_bvh(S, p, cx);
-    cx.box(2);
-    const float ll = node_lb(p, L.bmin, L.bmax), rl = node_lb(p, R.bmin, R.bmax);
-    const bool lfirst = ll <= rl;
-    leaf = lfirst ? L.leaf : R.leaf;
-    second = lfirst ? R.leaf : L.leaf;
-    second_lb = lfirst ? rl : ll;
-  }
-  return scene_distance_leaves(S, p, leaf, second, second_lb, cx);
 }
 
 // The primitive of DevFast::rec (a ground, usually), from the constant bank.
@@ -852,6 +823,28 @@ __device__ __forceinline__ Info pair_distance(const DevScene& S, F3 p, float l2,
   if (!(sqrtf(lfirst ? r2 : l2) <= a.d)) return a;
   const Info b{compact_at<true>(S, e1, p, cx), compact_ref(e1)};
   return b.d < a.d ? b : a;
+}
+
+// kFastLeaves: the nearer leaf, then the other when its box bound is not above
+// the distance found (the strictly-closer replace of bvh_distance_info); l and
+// r are the box bounds.  One evaluation site for both leaves.
+template <bool kStats>
+__device__ __forceinline__ Info leaves_distance(const DevScene& S, F3 p, float l, float r, Ctx<kStats>& cx) {
+  const DevFast& F = S.fast;
+  bool left = F.leaf[0] >= 0 && l <= r;
+  const float second_lb = left ? r : l;
+  Info cur{kInf, ftd::kNoRef};
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t e = left ? F.entry[0] : F.entry[1];
+    const int leaf = left ? F.leaf[0] : F.leaf[1];
+    const Info in = e != kNoPrim ? Info{compact_at<true>(S, e, p, cx), compact_ref(e)}
+                                 : eval_composite(S, leaf, __ldg(S.leaf_info + leaf), p, k == 0 ? kInf : cur.d, cx);
+    if (k == 0 || in.d < cur.d) cur = in;
+    if (F.leaf[0] < 0 || !(second_lb <= cur.d)) break;
+    left = !left;
+  }
+  return cur;
 }
 
 // kFastUnion: the nearest of the always-evaluated primitives (all of a small
@@ -913,29 +906,50 @@ __device__ __forceinline__ Info union_distance(const DevScene& S, F3 p, Ctx<kSta
   return best;
 }
 
-// The scene distance at p (Accelerator::distance_info): the short form of the
-// scene's kind inline in the march loops, every other scene out of line, so
-// that the loops' code stays small.
+// Scenes without a form of their own: one or two leaves, or the leaf walk.
 template <bool kStats>
+__device__ __forceinline__ Info general_distance(const DevScene& S, F3 p, Ctx<kStats>& cx) {
+  const DevFast& F = S.fast;
+  if (F.kind == kFastNone) return scene_distance_bvh(S, p, cx);
+  if (F.leaf[0] < 0) return leaves_distance(S, p, 0.0f, 0.0f, cx);
+  cx.box(2);
+  return leaves_distance(S, p, node_lb(p, F.bmin[0], F.bmax[0]), node_lb(p, F.bmin[1], F.bmax[1]), cx);
+}
+template <bool kStats>
+__device__ __noinline__ Info scene_distance_general(const DevScene& S, F3 p, Ctx<kStats>& cx) {
+  return general_distance(S, p, cx);
+}
+
+// What a march kernel is compiled for: scenes with a short form, scenes without
+// one (general), or any (mixed batches, statistics, paths: there the general
+// distance is a call).  In one kernel, the general distance inline made the
+// field's depth frame 4 % and a preview 4 to 6 % slower; behind a call, itself
+// calling the composite leaf's evaluator, a ground beside one boolean took 10
+// to 17 % longer than with its own kernel.
+enum Form : int { kFormAny = 0, kFormGeneral = 1, kFormShort = 2 };
+
+// The scene distance at p (Accelerator::distance_info).
+template <int kForm = kFormAny, bool kStats>
 __device__ __forceinline__ Info scene_distance_inl(const DevScene& S, F3 p, Ctx<kStats>& cx) {
   cx.eval();
   const DevFast& F = S.fast;
+  if (kForm == kFormGeneral) return general_distance(S, p, cx);
   if (F.kind == kFastUnion) return union_distance(S, p, cx);
-  if (F.kind == kFastNone) return scene_distance_general(S, p, cx);
+  if (kForm == kFormAny && F.kind <= kFastNone) return scene_distance_general(S, p, cx);
   if (F.entry[0] == kNoPrim) return eval_urtree(S, F.tree, p, kInf, cx);
   cx.box(2);
   const float l2 = ftd::aabb_lb2(p, F.bmin[0], F.bmax[0]), r2 = ftd::aabb_lb2(p, F.bmin[1], F.bmax[1]);
   return F.kind == kFastTree ? tree_and_prim(S, p, r2, l2, cx) : pair_distance(S, p, l2, r2, cx);
 }
 
-template <bool kStats>
+template <int kForm = kFormAny, bool kStats>
 __device__ __noinline__ Info scene_distance(const DevScene& S, F3 p, Ctx<kStats>& cx) {
-  return scene_distance_inl(S, p, cx);
+  return scene_distance_inl<kForm>(S, p, cx);
 }
 
-template <bool kStats>
+template <int kForm = kFormAny, bool kStats>
 __device__ __forceinline__ float scene_d(const DevScene& S, F3 p, Ctx<kStats>& cx) {
-  return scene_distance(S, p, cx).d;
+  return scene_distance<kForm>(S, p, cx).d;
 }
 
 // The same leaf-BVH walk reporting the winning hard-union leaf: the leaf whose
@@ -993,7 +1007,7 @@ struct HitOut {
   F3 normal;
 };
 
-template <bool kStats>
+template <int kForm, bool kStats>
 __device__ HitOut march(const DevScene& S, const RayParams& P, F3 o, F3 d, bool want_normal, Ctx<kStats>& cx) {
   HitOut h{0.0f, 0u, false, f3(0.0f, 0.0f, 0.0f)};
   float t0, t1;
@@ -1007,12 +1021,12 @@ __device__ HitOut march(const DevScene& S, const RayParams& P, F3 o, F3 d, bool 
   for (uint32_t s = 0; s < P.max_steps; ++s) {
     if (traveled > max_t) return h;
     cx.step();
-    Info info = scene_distance(S, o + d * traveled, cx);
+    Info info = scene_distance<kForm>(S, o + d * traveled, cx);
     if (fabsf(info.d) < eps) {
       float lo = prev, hi = traveled;
       for (int k = 0; k < 10; ++k) {
         float mid = 0.5f * (lo + hi);
-        float dm = fabsf(scene_d(S, o + d * mid, cx));
+        float dm = fabsf(scene_d<kForm>(S, o + d * mid, cx));
         if (dm < eps) hi = mid;
         else lo = mid;
       }
@@ -1020,13 +1034,13 @@ __device__ HitOut march(const DevScene& S, const RayParams& P, F3 o, F3 d, bool 
       if (want_normal) {
         // estimate_normal (R:4202-4215)
         float e = fmaxf(eps * 4.0f, 1.0e-5f);
-        float dx = scene_d(S, f3(pos.x + e, pos.y, pos.z), cx) - scene_d(S, f3(pos.x - e, pos.y, pos.z), cx);
-        float dy = scene_d(S, f3(pos.x, pos.y + e, pos.z), cx) - scene_d(S, f3(pos.x, pos.y - e, pos.z), cx);
-        float dz = scene_d(S, f3(pos.x, pos.y, pos.z + e), cx) - scene_d(S, f3(pos.x, pos.y, pos.z - e), cx);
+        float dx = scene_d<kForm>(S, f3(pos.x + e, pos.y, pos.z), cx) - scene_d<kForm>(S, f3(pos.x - e, pos.y, pos.z), cx);
+        float dy = scene_d<kForm>(S, f3(pos.x, pos.y + e, pos.z), cx) - scene_d<kForm>(S, f3(pos.x, pos.y - e, pos.z), cx);
+        float dz = scene_d<kForm>(S, f3(pos.x, pos.y, pos.z + e), cx) - scene_d<kForm>(S, f3(pos.x, pos.y, pos.z - e), cx);
         F3 nn = f3(dx, dy, dz);
         h.normal = ftd::len3(nn) > 1.0e-8f ? ftd::normalize3(nn) : f3(0.0f, 1.0f, 0.0f);
       }
-      Info fin = scene_distance(S, pos, cx);
+      Info fin = scene_distance<kForm>(S, pos, cx);
       h.t = hi;
       h.mat = surface_ids(S, fin.ref).y;
       h.hit = true;
@@ -1087,7 +1101,7 @@ __device__ __forceinline__ uint32_t batch_item(const BatchView& V, uint64_t g) {
   return lo;
 }
 
-template <bool kStats>
+template <bool kStats, int kForm>
 __global__ void __launch_bounds__(128) march_depth_kernel(const __grid_constant__ DevScene S,
                                                           const __grid_constant__ RayParams P, float* __restrict__ t_out,
                                                           uint8_t* __restrict__ mask_out,
@@ -1112,7 +1126,7 @@ __global__ void __launch_bounds__(128) march_depth_kernel(const __grid_constant_
     F3 dir = ftd::normalize3(fwd + rt * (ndc_x * P.tan_fov) + up * (ndc_y * P.tan_fov));
     dir = ftd::normalize3(dir);
     F3 o = f3(P.origin[0], P.origin[1], P.origin[2]);
-    HitOut h = march(S, P, o, dir, normal_out != nullptr, cx);
+    HitOut h = march<kForm>(S, P, o, dir, normal_out != nullptr, cx);
     size_t idx = (static_cast<size_t>(py) * P.width + px) * P.aa + s;
     t_out[idx] = h.hit ? h.t : 0.0f;
     mask_out[idx] = h.hit ? 1 : 0;
@@ -1183,7 +1197,7 @@ constexpr unsigned long long kMarchWallNs = 20ull * 1000000000ull;  // per warp
 // latency of its longest rays' evaluations and a 256x256 preview takes 0.42 ms
 // of march against 0.46 with six or eight blocks; the 512-primitive field at
 // 1920x1080 takes 12.7, 12.7 and 11.8 ms (refilling at 8 idle lanes).
-template <bool kStats, bool kBricks, bool kBatch>
+template <bool kStats, bool kBricks, bool kBatch, int kForm = kFormAny>
 __global__ void __launch_bounds__(128, 5) march_depth_persistent(
     const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ DevBricks B0,
     const __grid_constant__ BatchView V,
@@ -1380,7 +1394,7 @@ __global__ void __launch_bounds__(128, 5) march_depth_persistent(
     } else {
       q = pos;
     }
-    Info info = scene_distance_inl(S, q, cx);
+    Info info = scene_distance_inl<kForm>(S, q, cx);
 
     if (phase == kMarch) {
       if (fabsf(info.d) < eps) {

@@ -377,6 +377,21 @@ ft_status upload_scene(ft_scene* sc) {
       n_listed = static_cast<int32_t>(im.leaves.size()) - n_always;
     }
   }
+  // One or two leaves of other kinds: the root's children, or the only leaf
+  // second, with a record where a leaf is a primitive.
+  const bool few = im.leaves.size() <= 2 && im.fast_tree < 0 && !im.fast_union;
+  int32_t few_leaf[2] = {-1, 0};
+  uint32_t few_entry[2] = {kNoPrim, kNoPrim};
+  if (few && im.leaves.size() == 2) {
+    few_leaf[0] = im.bvh[im.bvh[im.bvh_root].lhs].leaf;
+    few_leaf[1] = im.bvh[im.bvh[im.bvh_root].rhs].leaf;
+  }
+  for (int k = 0; few && k < 2; ++k) {
+    if (few_leaf[k] < 0 || im.leaves[few_leaf[k]].kind != ftgpu::kLeafPrim) continue;
+    const ftgpu::CompactPrim c = ftgpu::compact_prim(im, im.leaves[few_leaf[k]].node, static_cast<uint32_t>(few_leaf[k]));
+    few_entry[k] = static_cast<uint32_t>(cprims.size()) | (c.leaf & ftd::kRareFlag);
+    cprims.push_back(c);
+  }
   ftgpu::build_far_tree(im, cprims, n_always, n_listed, &far_nodes, &far_entries);  // (a union has no trees before it)
   auto listed_box = [&](float mn[3], float mx[3]) {
     for (int k = n_always; k < n_always + n_listed; ++k) {
@@ -524,6 +539,7 @@ ft_status upload_scene(ft_scene* sc) {
   DevFast& F = d.fast;
   F.kind = kFastNone;
   F.entry[0] = F.entry[1] = kNoPrim;
+  F.leaf[0] = F.leaf[1] = -1;
   auto box = [&](int k, const float* mn, const float* mx) {
     std::memcpy(F.bmin[k], mn, sizeof(F.bmin[k]));
     std::memcpy(F.bmax[k], mx, sizeof(F.bmax[k]));
@@ -557,6 +573,14 @@ ft_status upload_scene(ft_scene* sc) {
       for (size_t k = 0; k < jobs.size(); ++k) (k == 0 ? F.tree.fine : F.tree.outer) = dev_grid(jobs[k]);
     }
   }
+  if (few) {
+    F.kind = kFastLeaves;
+    for (int k = 0; k < 2; ++k) {
+      F.entry[k] = few_entry[k];
+      F.leaf[k] = few_leaf[k];
+      if (few_leaf[k] >= 0) box(k, im.leaves[few_leaf[k]].bmin, im.leaves[few_leaf[k]].bmax);
+    }
+  }
   // (without any grid the far walk would meet points inside the solids, where
   // the leaf walk's order counts)
   if (F.kind == kFastUnion && !F.all && F.tree.fine.dims[0] <= 0 && F.tree.outer.dims[0] <= 0) F.kind = kFastNone;
@@ -566,11 +590,13 @@ ft_status upload_scene(ft_scene* sc) {
   FT_CUDA_TRY(cudaMalloc(&sc->d_stats, kStatWords * sizeof(unsigned long long)), "cudaMalloc(stats)");
   int sms = 0, per_sm = 0;
   FT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sc->device), "sm count");
-  FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, false, false>, 128, 0),
+  FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, false, false, kFormShort>, 128,
+                                                            0),
               "occupancy");
   sc->persistent_blocks = std::max(1, sms * std::max(per_sm, 1));
   sc->sms = std::max(1, sms);
-  FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, true, false>, 128, 0),
+  FT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_depth_persistent<false, true, false, kFormShort>, 128,
+                                                            0),
               "occupancy");
   sc->persistent_blocks_bricks = std::max(1, sms * std::max(per_sm, 1));
   // Renders run on any stream, also on ones that do not wait for this one: the
@@ -694,14 +720,14 @@ ft_status launch_depth(ft_scene* sc, const RayParams& P, cudaStream_t st, bool s
     return FT_OK;
   }
   int ev = prof_begin(sc, st, FT_KERNEL_DEPTH_MARCH);
-  if (stats && bricks)
-    march_depth_persistent<true, true, false><<<grid, 128, 0, st>>>(sc->dev, P, B, BatchView{}, t, mask, mat, normal, st_ptr, counter);
-  else if (stats)
-    march_depth_persistent<true, false, false><<<grid, 128, 0, st>>>(sc->dev, P, B, BatchView{}, t, mask, mat, normal, st_ptr, counter);
-  else if (bricks)
-    march_depth_persistent<false, true, false><<<grid, 128, 0, st>>>(sc->dev, P, B, BatchView{}, t, mask, mat, normal, st_ptr, counter);
-  else
-    march_depth_persistent<false, false, false><<<grid, 128, 0, st>>>(sc->dev, P, B, BatchView{}, t, mask, mat, normal, st_ptr, counter);
+  const bool general = sc->dev.fast.kind <= kFastNone;
+  auto* march = stats && bricks ? march_depth_persistent<true, true, false>
+                : stats         ? march_depth_persistent<true, false, false>
+                : bricks ? (general ? march_depth_persistent<false, true, false, kFormGeneral>
+                                    : march_depth_persistent<false, true, false, kFormShort>)
+                         : (general ? march_depth_persistent<false, false, false, kFormGeneral>
+                                    : march_depth_persistent<false, false, false, kFormShort>);
+  march<<<grid, 128, 0, st>>>(sc->dev, P, B, BatchView{}, t, mask, mat, normal, st_ptr, counter);
   prof_end(sc, st, ev);
   FT_CUDA_TRY(cudaGetLastError(), "march_depth_persistent launch");
   return FT_OK;
@@ -745,6 +771,7 @@ struct BatchPart {
   uint64_t n_samples = 0;
   std::vector<uint64_t> out_first;
   int blocks = 1;
+  bool general = false;  // no scene has a short form
   BatchView view() const {
     BatchView v{};
     v.scenes = d_scenes;
@@ -898,12 +925,12 @@ ft_status batch_apply_tuning(ft_batch* b) {
   const BatchPart& D = b->part[0];
   const BatchPart& T = b->part[1];
   if (!D.items.empty()) {
-    if (b->bricks)
-      march_depth_persistent<false, true, true><<<D.blocks, 128, 0, b->stream>>>(
-          DevScene{}, RayParams{}, DevBricks{}, D.view(), b->d_t, b->d_mask, nullptr, nullptr, nullptr, b->d_counters);
-    else
-      march_depth_persistent<false, false, true><<<D.blocks, 128, 0, b->stream>>>(
-          DevScene{}, RayParams{}, DevBricks{}, D.view(), b->d_t, b->d_mask, nullptr, nullptr, nullptr, b->d_counters);
+    auto* march = b->bricks ? (D.general ? march_depth_persistent<false, true, true, kFormGeneral>
+                                         : march_depth_persistent<false, true, true>)
+                            : (D.general ? march_depth_persistent<false, false, true, kFormGeneral>
+                                         : march_depth_persistent<false, false, true>);
+    march<<<D.blocks, 128, 0, b->stream>>>(DevScene{}, RayParams{}, DevBricks{}, D.view(), b->d_t, b->d_mask, nullptr,
+                                           nullptr, nullptr, b->d_counters);
   }
   if (!T.items.empty()) {
     // the Whitted items as a wavefront: one march, shade and shadow kernel
@@ -914,22 +941,22 @@ ft_status batch_apply_tuning(ft_batch* b) {
     cudaMemsetAsync(c, 0, kWfCounters * sizeof(unsigned long long), b->stream);
     const unsigned grid = static_cast<unsigned>(T.blocks);
     const unsigned mgrid = static_cast<unsigned>(b->sms * 6), sgrid = static_cast<unsigned>(b->sms * 8);
+    auto* march = T.general ? wf_march_persistent<true, false, kFormGeneral> : wf_march_persistent<true, false>;
+    auto* shadow = T.general ? wf_shadow_persistent<true, false, kFormGeneral> : wf_shadow_persistent<true, false>;
     wf_primary_batch_kernel<<<grid, 128, 0, b->stream>>>(V, b->wf_jobs[0], c);
     for (uint32_t level = 0; level < b->wf_levels; ++level) {
       const int cur = static_cast<int>(level & 1), nxt = 1 - cur;
       cudaMemsetAsync(c + nxt, 0, sizeof(unsigned long long), b->stream);
       cudaMemsetAsync(c + 2, 0, sizeof(unsigned long long), b->stream);
       cudaMemsetAsync(c + 4, 0, 2 * sizeof(unsigned long long), b->stream);
-      wf_march_persistent<true, false><<<mgrid, 128, 0, b->stream>>>(DevScene{}, RayParams{}, V, b->wf_jobs[cur],
-                                                                     c + cur, b->wf_jobs_cap[cur], b->wf_hits,
-                                                                     b->d_srgb, c + 4, c + 6, nullptr);
+      march<<<mgrid, 128, 0, b->stream>>>(DevScene{}, RayParams{}, V, b->wf_jobs[cur], c + cur, b->wf_jobs_cap[cur],
+                                          b->wf_hits, b->d_srgb, c + 4, c + 6, nullptr);
       WQueues Q{b->d_srgb, b->wf_jobs[nxt], c + nxt, b->wf_jobs_cap[nxt], b->wf_shadows, c + 2,
                 b->wf_shadows_cap, reinterpret_cast<unsigned int*>(c + 3), 0};
       wf_shade_batch_kernel<<<grid, 128, 0, b->stream>>>(V, T.d_max_depth, b->wf_jobs[cur], c + cur,
                                                          b->wf_jobs_cap[cur], b->wf_hits, Q);
-      wf_shadow_persistent<true, false><<<sgrid, 128, 0, b->stream>>>(DevScene{}, RayParams{}, V, b->wf_shadows,
-                                                                      c + 2, b->wf_shadows_cap, b->d_srgb, c + 5,
-                                                                      c + 6, nullptr);
+      shadow<<<sgrid, 128, 0, b->stream>>>(DevScene{}, RayParams{}, V, b->wf_shadows, c + 2, b->wf_shadows_cap,
+                                           b->d_srgb, c + 5, c + 6, nullptr);
     }
   }
   {
@@ -1025,16 +1052,18 @@ ft_status trace_wavefront(ft_scene* sc, const RayParams& P, uint32_t max_depth, 
   FT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sc->device), "sm count");
   // statistics runs take the precompiled counting variants; the run-time
   // compiled kernels, when present, serve every other trace
-  const bool stats = kind_stats != nullptr;
+  const bool stats = kind_stats != nullptr, general = sc->dev.fast.kind <= kFastNone;
   const void* k_march = stats ? reinterpret_cast<const void*>(wf_march_persistent<false, true>)
                         : sc->jit_wf[0] ? reinterpret_cast<const void*>(sc->jit_wf[0])
-                                        : reinterpret_cast<const void*>(wf_march_persistent<false, false>);
+                        : general      ? reinterpret_cast<const void*>(wf_march_persistent<false, false, kFormGeneral>)
+                                       : reinterpret_cast<const void*>(wf_march_persistent<false, false, kFormShort>);
   const void* k_shade = stats ? reinterpret_cast<const void*>(wf_shade_kernel<true>)
                         : sc->jit_wf[1] ? reinterpret_cast<const void*>(sc->jit_wf[1])
                                         : reinterpret_cast<const void*>(wf_shade_kernel<false>);
   const void* k_shadow = stats ? reinterpret_cast<const void*>(wf_shadow_persistent<false, true>)
                          : sc->jit_wf[2] ? reinterpret_cast<const void*>(sc->jit_wf[2])
-                                         : reinterpret_cast<const void*>(wf_shadow_persistent<false, false>);
+                         : general      ? reinterpret_cast<const void*>(wf_shadow_persistent<false, false, kFormGeneral>)
+                                        : reinterpret_cast<const void*>(wf_shadow_persistent<false, false, kFormShort>);
   unsigned long long* st_march = stats ? kind_stats[0] : nullptr;
   unsigned long long* st_shade = stats ? kind_stats[1] : nullptr;
   unsigned long long* st_shadow = stats ? kind_stats[2] : nullptr;
@@ -1329,8 +1358,9 @@ ft_status ft_render_depth_preview_noalloc(ft_scene* sc, const ft_render_options*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   RayParams P = make_params(sc, *options, aa);
   uint64_t blocks = (P.n_items + 127) / 128;
-  march_depth_kernel<false><<<static_cast<unsigned>(blocks), 128, 0, st>>>(sc->dev, P, t, mask, nullptr, nullptr,
-                                                                           nullptr);
+  auto* march = sc->dev.fast.kind <= kFastNone ? march_depth_kernel<false, kFormGeneral>
+                                               : march_depth_kernel<false, kFormShort>;
+  march<<<static_cast<unsigned>(blocks), 128, 0, st>>>(sc->dev, P, t, mask, nullptr, nullptr, nullptr);
   FT_CUDA_TRY(cudaGetLastError(), "march_depth_kernel launch");
   uint32_t np = static_cast<uint32_t>(pixels);
   depth_rgb8_kernel<<<(np + 255) / 256, 256, 0, st>>>(t, mask, np, aa, options->max_dist, rgb8_out);
@@ -1891,6 +1921,7 @@ ft_status ft_batch_create(const ft_batch_item* items, uint32_t n, uint32_t flags
       bricks_v.push_back(b->items[it].scene->bricks);
       depth.push_back(std::max(b->items[it].max_depth, 1u));
     }
+    part.general = std::all_of(scenes.begin(), scenes.end(), [](const DevScene& d) { return d.fast.kind <= kFastNone; });
     FT_CUDA_TRY(cudaMalloc(&part.d_scenes, m * sizeof(DevScene)), "cudaMalloc(batch scenes)");
     FT_CUDA_TRY(cudaMalloc(&part.d_params, m * sizeof(RayParams)), "cudaMalloc(batch params)");
     FT_CUDA_TRY(cudaMalloc(&part.d_bricks, m * sizeof(DevBricks)), "cudaMalloc(batch bricks)");
@@ -2144,8 +2175,10 @@ ft_status ft_render_views(ft_scene* sc, const ft_view* views, uint32_t n_views, 
   FT_CUDA_TRY(tmp.alloc(&d_counters, kViewCounters), "cudaMalloc(counters)");
   FT_CUDA_TRY(cudaMemsetAsync(d_counters, 0, kViewCounters * sizeof(unsigned long long), st), "memset");
   const uint64_t n_work = items * n_views;
-  views_march_persistent<false><<<view_blocks(sc, n_work), 128, 0, st>>>(sc->dev, d_views, items, 0, n_work, tau, t, m,
-                                                                         sil, nullptr, nullptr, nullptr, d_counters);
+  auto* march = sc->dev.fast.kind <= kFastNone ? views_march_persistent<false, kFormGeneral>
+                                               : views_march_persistent<false, kFormShort>;
+  march<<<view_blocks(sc, n_work), 128, 0, st>>>(sc->dev, d_views, items, 0, n_work, tau, t, m, sil, nullptr, nullptr,
+                                                 nullptr, d_counters);
   FT_CUDA_TRY(cudaGetLastError(), "views_march_persistent launch");
   unsigned long long march_flags = 0;
   FT_CUDA_TRY(cudaMemcpyAsync(&march_flags, d_counters + 1, sizeof(march_flags), cudaMemcpyDeviceToHost, st),
@@ -2250,8 +2283,10 @@ ft_status ft_render_backward(ft_scene* sc, const ft_view* views, uint32_t n_view
     FT_CUDA_TRY(cudaMemsetAsync(d_counters, 0, sizeof(unsigned long long), st), "memset");
     FT_CUDA_TRY(cudaMemsetAsync(d_counters + 2, 0, 2 * sizeof(unsigned long long), st), "memset");
     const unsigned grid = view_blocks(sc, n);
-    views_march_persistent<true><<<grid, 128, 0, st>>>(sc->dev, d_views, items, first, n, tau, nullptr, nullptr,
-                                                       nullptr, a, b, d_rays, d_counters);
+    auto* march = sc->dev.fast.kind <= kFastNone ? views_march_persistent<true, kFormGeneral>
+                                                 : views_march_persistent<true, kFormShort>;
+    march<<<grid, 128, 0, st>>>(sc->dev, d_views, items, first, n, tau, nullptr, nullptr, nullptr, a, b, d_rays,
+                                d_counters);
     FT_CUDA_TRY(cudaGetLastError(), "views_march_persistent launch");
     views_adjoint_kernel<<<grid, 128, shared_acc ? smem : 0, st>>>(sc->dev, d_views, items, n, tau, T, d_rays,
                                                                    d_counters, d_grad, shared_acc, d_bad);
@@ -2283,16 +2318,25 @@ ft_status ft_scene_jit(ft_scene* sc, ft_jit_info* info) {
   const ftgpu::SceneImage& im = sc->img;
   ft_jit_info out{};
   out.programs = static_cast<uint32_t>(im.programs.size());
-  std::string src = "// scene module compiled at run time\n#include \"ft_kernels.cuh\"\nnamespace {\n" +
+  const bool general = sc->dev.fast.kind <= kFastNone;
+  std::string src = "// scene module compiled at run time" + std::string(general ? ": general form" : ": short form") +
+                    "\n#include \"ft_kernels.cuh\"\nnamespace {\n" +
                     ftgpu::jit_hook_source(im.programs.data(), static_cast<uint32_t>(im.programs.size()),
                                            im.instrs.data()) +
                     "}  // namespace\n";
   out.source_bytes = src.size();
   constexpr int kJitKernels = 5;
-  static const char* const kExprs[kJitKernels] = {"march_depth_persistent<false, false, false>",
-                                                  "march_depth_persistent<false, true, false>",
-                                                  "wf_march_persistent<false, false>", "wf_shade_kernel<false>",
-                                                  "wf_shadow_persistent<false, false>"};
+  static const char* const kShortExprs[kJitKernels] = {"march_depth_persistent<false, false, false, kFormShort>",
+                                                       "march_depth_persistent<false, true, false, kFormShort>",
+                                                       "wf_march_persistent<false, false, kFormShort>",
+                                                       "wf_shade_kernel<false>",
+                                                       "wf_shadow_persistent<false, false, kFormShort>"};
+  static const char* const kGeneralExprs[kJitKernels] = {"march_depth_persistent<false, false, false, kFormGeneral>",
+                                                         "march_depth_persistent<false, true, false, kFormGeneral>",
+                                                         "wf_march_persistent<false, false, kFormGeneral>",
+                                                         "wf_shade_kernel<false>",
+                                                         "wf_shadow_persistent<false, false, kFormGeneral>"};
+  const char* const* kExprs = general ? kGeneralExprs : kShortExprs;
   struct Module {
     std::vector<char> cubin;
     std::string lowered[kJitKernels];
@@ -2321,7 +2365,7 @@ ft_status ft_scene_jit(ft_scene* sc, ft_jit_info* info) {
     nvrtcResult r = nvrtcCreateProgram(&prog, src.c_str(), "ft_scene_jit.cu", nh, texts.data(), names.data());
     if (r != NVRTC_SUCCESS) return ftcommon::fail(FT_ERR_JIT, std::string("nvrtcCreateProgram: ") + nvrtcGetErrorString(r));
     std::unique_ptr<nvrtcProgram, void (*)(nvrtcProgram*)> guard(&prog, [](nvrtcProgram* p) { nvrtcDestroyProgram(p); });
-    for (const char* e : kExprs) nvrtcAddNameExpression(prog, e);
+    for (int k = 0; k < kJitKernels; ++k) nvrtcAddNameExpression(prog, kExprs[k]);
     int major = 0, minor = 0;
     FT_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, sc->device), "device arch");
     FT_CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, sc->device), "device arch");

@@ -242,7 +242,7 @@ __device__ __noinline__ void wf_add_miss(const DevScene& S, const RayParams& P, 
 // (the launch is five per SM): on the 512-primitive field's depth-6 trace,
 // 70 ms of march per frame against 73 with six and 71 with eight, and a
 // 353x199 trace, bound by its longest rays' latency, 2.0 against 2.2 ms.
-template <bool kBatch, bool kStats>
+template <bool kBatch, bool kStats, int kForm = kFormAny>
 __global__ void __launch_bounds__(128, 5) wf_march_persistent(
     const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ BatchView V,
                                                               const WJob* __restrict__ jobs,
@@ -336,12 +336,13 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(
     // nearest primitive, whose record holds its leaf; the general walk's final
     // lookup is its own (a lane in its final phase would keep the others
     // waiting through a second evaluation).
-    const bool final = phase == kWfFinal, general = S.fast.kind == kFastNone;
+    const bool final = phase == kWfFinal,
+               general = kForm == kFormGeneral || (kForm == kFormAny && S.fast.kind <= kFastNone);
     WHit h{};
     Info info{0.0f, ftd::kNoRef};
     if (!(final && general)) {
       const unsigned long long boxes = kStats ? cx.c.boxes : 0ull;
-      info = scene_distance_inl(S, q, cx);
+      info = scene_distance_inl<kForm>(S, q, cx);
       if (kStats && final) cx.c.boxes = boxes;  // (the lookup of a hit's leaf is not counted as a cull)
     }
     if (final) {
@@ -400,22 +401,28 @@ __global__ void __launch_bounds__(128, 5) wf_march_persistent(
 }
 
 // A step of shadow_visibility (R:4706-4733): the leaf-box lower bound when it
-// exceeds max(8 eps, 0.02), else the exact distance.  The short scene forms
-// compute their box bounds once for both; a hard union's bound is 0 inside the
-// box of any primitive that is evaluated at every point (a ground).
-template <bool kStats>
+// exceeds max(8 eps, 0.02), else the exact distance.  The short scene forms,
+// and one or two leaves, compute their box bounds once for both; a hard
+// union's bound is 0 inside the box of any primitive that is evaluated at
+// every point (a ground).
+template <int kForm, bool kStats>
 __device__ __forceinline__ float shadow_step_h(const DevScene& S, F3 p, float eps, Ctx<kStats>& cx) {
   const DevFast& F = S.fast;
   const float least = fmaxf(eps * 8.0f, 0.02f);
   float l2 = kInf, r2 = kInf, lower;
-  if (F.kind == kFastTree || F.kind == kFastPair) {
+  if (kForm == kFormGeneral && F.kind == kFastLeaves) {
+    if (F.leaf[0] >= 0) l2 = ftd::aabb_lb2(p, F.bmin[0], F.bmax[0]);
+    r2 = ftd::aabb_lb2(p, F.bmin[1], F.bmax[1]);
+    cx.box(F.leaf[0] >= 0 ? 3 : 1);
+    lower = sqrtf(fminf(l2, r2));
+  } else if (kForm != kFormGeneral && (F.kind == kFastTree || F.kind == kFastPair)) {
     if (F.entry[0] != kNoPrim) l2 = ftd::aabb_lb2(p, F.bmin[0], F.bmax[0]);
     r2 = ftd::aabb_lb2(p, F.bmin[1], F.bmax[1]);
     cx.box(F.entry[0] == kNoPrim ? 1 : 3);
     lower = sqrtf(fminf(l2, r2));
   } else {
     bool known = false;
-    if (F.kind == kFastUnion) {
+    if (kForm != kFormGeneral && F.kind == kFastUnion) {
       for (int i = 0; i < F.n_always; ++i) {
         const DevNode& n = S.nodes[__float_as_int(__ldg(S.cprims + 3 * i + 2).z)];
         cx.box();
@@ -428,8 +435,10 @@ __device__ __forceinline__ float shadow_step_h(const DevScene& S, F3 p, float ep
   if (lower > least) return lower;
   cx.eval();
   Info h;
-  if (F.kind == kFastUnion) h = union_distance(S, p, cx);
-  else if (F.kind == kFastNone) h = scene_distance_general(S, p, cx);
+  if (kForm == kFormGeneral)
+    h = F.kind == kFastNone ? scene_distance_bvh(S, p, cx) : leaves_distance(S, p, sqrtf(l2), sqrtf(r2), cx);
+  else if (F.kind == kFastUnion) h = union_distance(S, p, cx);
+  else if (kForm == kFormAny && F.kind <= kFastNone) h = scene_distance_general(S, p, cx);
   else if (F.kind == kFastPair) h = pair_distance(S, p, l2, r2, cx);
   else if (F.entry[0] == kNoPrim) h = eval_urtree(S, F.tree, p, kInf, cx);
   else h = tree_and_prim(S, p, r2, l2, cx);
@@ -438,7 +447,7 @@ __device__ __forceinline__ float shadow_step_h(const DevScene& S, F3 p, float ep
 
 // shadow_visibility (R:4706-4733) of every queued shadow job, one step per
 // iteration; the radiance gets contribution x visibility.
-template <bool kBatch, bool kStats>
+template <bool kBatch, bool kStats, int kForm = kFormAny>
 __global__ void __launch_bounds__(128, 8) wf_shadow_persistent(
     const __grid_constant__ DevScene S0, const __grid_constant__ RayParams P0, const __grid_constant__ BatchView V,
                                                                const WShadow* __restrict__ shadows,
@@ -494,7 +503,7 @@ __global__ void __launch_bounds__(128, 8) wf_shadow_persistent(
       continue;
     }
     F3 p = o + d * t;
-    const float h = shadow_step_h(S, p, eps, cx);
+    const float h = shadow_step_h<kForm>(S, p, eps, cx);
     if (h < eps * 4.0f) {
       finish(0.0f);
       continue;

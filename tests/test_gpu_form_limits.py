@@ -334,3 +334,43 @@ def test_adjoint_in_chunks_of_rays():
     parts = sum(ps.backward(vs[k:k + 1], opts, w[0][k:k + 1], w[1][k:k + 1]) for k in range(5))
     assert np.abs(whole).max() > 0
     assert np.abs(whole - parts).max() <= 1e-9 * np.abs(parts).max()
+
+
+LEAVES = {"boolean": "let {n} = (Sphere {{ radius: 0.8, pos: vec3({x}, 0.6, 0) }}) - "
+                     "(Box {{ size: vec3(0.9, 0.9, 0.9), pos: vec3({x}, 1.0, -0.3) }});",
+          "prism": "let {n} = ExtrudePolygon {{ sides: 3, radius: 0.7, height: 0.8, pos: vec3({x}, 0.5, 0) }};",
+          "turned": "let {n} = Box {{ size: vec3(0.9, 0.5, 0.7), round: 0.1, pos: vec3({x}, 0.7, 0), rot: vec3(20, 30, 10) }};",
+          "hooked": "let {n} = Sphere {{ radius: 0.6, pos: vec3({x}, 0.6, 0), "
+                    "distance_post: fn(d, p) {{ return abs(d) - 0.05; }} }};",
+          "sphere": "let {n} = Sphere {{ radius: 0.6, pos: vec3({x}, 0.6, 0) }};"}
+
+
+@pytest.mark.parametrize("kinds", [("boolean",), ("hooked",), ("prism",), ("boolean", "sphere"), ("sphere", "boolean"),
+                                   ("prism", "sphere"), ("prism", "prism"), ("hooked", "turned"), ("boolean", "hooked")])
+def test_scenes_of_one_or_two_leaves(kinds):
+    """Every pairing of leaf kinds in the short form of one or two leaves:
+    distances around the scene, and a depth frame and a trace whose hits find
+    their leaves, against the f32 oracle."""
+    lines = [LEAVES[k].format(n=f"l{i}", x=-0.9 + 1.8 * i) for i, k in enumerate(kinds)]
+    st = ft.parse_and_eval(LIGHTS + "\n".join(lines) + "\nlet scene = " + " + ".join(f"l{i}" for i in range(len(kinds))) + ";\n")
+    pts = np.concatenate([_points(8000, r) for r in (1.5, 6.0)])
+    ref, _, _ = oracle.distance(st, pts, accel=1, precision=32)
+    err = np.abs(_distances(st, pts) - ref)
+    assert (err > 1e-5 * np.maximum(1.0, np.abs(ref))).sum() <= 2, (float(err.max()), pts[err.argmax()])
+    opts = ft.RenderOptions(width=96, height=64, max_steps=256, max_dist=30.0, epsilon=1e-4, step_scale=0.7)
+    img = ft.render_depth(st, opts, ft.AccelMode.Bvh, 1, want_material=True)
+    t, m, mat, _, _ = oracle.render_depth(st, opts, 1, 1, 32)
+    both = (img.mask == 1) & (m == 1)
+    assert (img.mask == m).mean() >= 0.999 and both.mean() > 0.02
+    assert (np.abs(img.t[both] - t[both]) <= 1e-4).mean() >= 0.999 and (img.material[both] == mat[both]).all()
+    lin, _ = ft.render_trace(st, opts, ft.AccelMode.Bvh, 1, 2)
+    rad, _, _ = oracle.render_trace(st, opts, 1, 1, 2, 32)
+    assert radiance_rmse(lin, rad) <= 1e-3, radiance_rmse(lin, rad)
+    # the same frames from a batch of such scenes alone, and mixed with a scene of a short form
+    ball = ft.parse_and_eval(LIGHTS + "let scene = Sphere { radius: 0.5, pos: vec3(0, 0.6, 0) };\n")
+    for others in ([], [ball]):
+        b = ft.Batch([(x, opts, 1, depth) for x in [st, *others] for depth in (0, 2)])
+        b.launch()
+        assert np.array_equal(b.read(0)["t"], img.t) and np.array_equal(b.read(0)["mask"], img.mask)
+        assert np.allclose(b.read(1)["rgb"], lin, rtol=1e-3, atol=1e-4)  # the sums' order varies
+        b.close()
