@@ -34,8 +34,10 @@ FT_DEV F3 normalize3(F3 a) {
 }
 
 // normalize3 with its multiply-adds written out, the squares summed x or y
-// first (an ulp of a primary ray moves a silhouette pixel, so each kernel
-// keeps its order whatever the compiler contracts).
+// first.  A primary ray is normalised twice; the kernels differ in the order of
+// the second time only, by an ulp of the ray's length, and each keeps the one
+// its outputs have had.  (What leads up to the first is contracted as the
+// compiler chooses.)
 template <bool kYFirst>
 FT_DEV F3 normalize3_fma(F3 a) {
   const float u = kYFirst ? a.y : a.x, v = kYFirst ? a.x : a.y;

@@ -336,7 +336,8 @@ __device__ __noinline__ bool urtree_backprop_full(const DevScene& S, int ti, F3 
 // whole derivative is the nearest primitive's.  So the candidates of the
 // point's cell replace the fold of all primitives and its two arrays of n
 // floats in local memory, which bound the adjoint.  With the marches below, a
-// fitting step of 64 primitives and 32 views at 256^2 takes 14 ms, against 89.
+// fitting step of 64 primitives and 32 views at 256^2 takes 10.9 ms, against
+// 183 with the full fold and a thread per ray.
 //
 // The near primitives are joined as in ur_fold_many with every subtree's value
 // kept (ids 0..nn-1 the primitives in order, then the joins), and the adjoints

@@ -25,8 +25,8 @@
 //
 // Bound by the distance evaluations of the block's primitives (a few million
 // for 512 primitives).  Opening the 512-primitive field and rendering its
-// 800x600 preview takes 12 ms, against 38 ms with the lists built by 16 host
-// threads and copied.
+// 800x600 preview takes 8.4 ms; it took 38 when 16 host threads built the lists
+// and a slower march rendered it.
 //
 // Included by ft_kernels.cuh (precompiled only).
 #pragma once

@@ -590,7 +590,7 @@ __device__ __forceinline__ bool grid_cell(const DevGrid& g, F3 p, int* cell) {
 // primitive) and the branches between them, so each is one vector load of a
 // compact record and the distance has no branch.  With the scene's header in
 // the constant bank, the 512-primitive field's depth frame (1920x1080, 2x2)
-// takes 11.9 ms, against 29.8 ms with scalar loads from 128-byte nodes, a box
+// takes 10.6 ms, against 29.8 ms with scalar loads from 128-byte nodes, a box
 // test per candidate and parent-link folds.
 //
 // The tree's value at p, exact where it is below `cutoff`: the candidates of

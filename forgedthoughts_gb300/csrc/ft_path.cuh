@@ -444,8 +444,8 @@ constexpr uint32_t kPathStopped = 0x80000000u;
 // A path is a serial chain of distance evaluations and its length varies from
 // one bounce to max_bounces, so a frame needs many of them in flight: a thread
 // per pixel taking its samples in turn left 3 warps on a scheduler and the
-// longest pixel to wait for (320x180, 16 spp: 88 ms, now 50, and
-// 45 with ten blocks per SM instead of the compiler's five).
+// longest pixel to wait for (320x180, 16 spp: 88 ms; 50 with a path per thread,
+// 41 to 45 with ten blocks per SM instead of the compiler's five).
 __global__ void __launch_bounds__(128, 10) path_sample_kernel(const __grid_constant__ DevScene S,
                                                           const __grid_constant__ RayParams P, uint32_t max_bounces,
                                                           uint32_t first, uint32_t n, uint64_t first_pixel,

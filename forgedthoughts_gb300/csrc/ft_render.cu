@@ -307,12 +307,18 @@ DevGrid dev_grid(const GridJob& j) {
   return g;
 }
 
-// Most leaves of a hard union that are all evaluated at every point.
+// Most leaves of a hard union that are all evaluated at every point: a 64x64
+// preview of a ground and 5 spheres takes 0.46 ms with all evaluated and 0.44
+// with grids, of 8 spheres 0.58 and 0.48, of 40 1.49 and 0.51; below that the
+// grids' creation (0.1 ms) is saved.
 constexpr size_t kBruteLeaves = 4;
 
 // Grids of a hard union's listed primitives, whose boxes fill mn..mx: a fine
 // one over that box widened by a tenth, and a coarser one half an extent wider
-// around it.  Both end on their own entry caps.
+// around it.  With a quarter of the cells 2000 spread spheres' trace (512x288)
+// takes 10.1 ms instead of 7.2 and their creation 9.6 instead of 8.0, as a
+// block of cells then tests more candidates.  Creation and one 64x64 frame
+// together take less than the leaf walk's frame (8.6 against 10.7 ms there).
 void union_grids(const float mn[3], const float mx[3], int32_t first, int32_t n, std::vector<GridJob>* jobs) {
   const float widest = std::max({mx[0] - mn[0], mx[1] - mn[1], mx[2] - mn[2]});
   for (int k = 0; k < 2; ++k) {

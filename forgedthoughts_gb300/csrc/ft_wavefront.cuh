@@ -190,7 +190,9 @@ __device__ __forceinline__ uint32_t sample_item(const BatchView& V, uint64_t sam
 // (one atomic per warp) once at least kWfRefill lanes are idle: setting up a
 // ray is several hundred instructions whose cost the waiting lanes share, so
 // few large refills beat keeping the lanes full (1920x1080 depth of the
-// 512-primitive field: 14.8 ms at 4, 12.7 at 8, 12.0 at 16, 11.1 at 24).  With kBatch
+// 512-primitive field: 14.8 ms at 4, 12.7 at 8, 12.0 at 16, 11.1 at 24; where an
+// evaluation costs far more it makes no difference, 64 interpreted hooked
+// shells at 480x270: 26.4, 26.4, 26.4, 26.3).  With kBatch
 // each job's render (scene, parameters) is looked up from its sample index.
 // Self-checks as in march_depth_persistent: a job may take at most
 // max_steps + 64 iterations, a warp at most kMarchWallNs; a lane past either

@@ -635,7 +635,7 @@ class Builder {
     // grid, hence at least 2r from every primitive box: each cell lists the
     // primitives that can be the nearest, sorted by gap, as above (a walk of
     // the tree's BVH from such points tests about six times as many boxes).
-    // Points outside both grids take the tree BVH.
+    // Points outside both grids take the far walk.
     const double widen = 0.5 * std::max({ext[0], ext[1], ext[2]});
     Box outer = all;
     for (int a = 0; a < 3; ++a) {

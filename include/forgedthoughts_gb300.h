@@ -427,9 +427,12 @@ void ft_scene_desc_free(ft_scene_desc* desc);
 ft_status ft_scene_create(const ft_scene_desc* desc, ft_scene** out);
 void ft_scene_destroy(ft_scene* scene);
 
-/* Host-only summary of the culling structures ft_scene_create would build for
- * `desc` (no device needed): hard-union leaves by evaluation kind, the
- * union_round trees and their candidate grids. */
+/* Host-only summary of `desc` (no device needed): hard-union leaves by
+ * evaluation kind, the union_round trees, and candidate grids of these trees
+ * with the cells ft_scene_create takes.  The lists are a host restatement with
+ * looser bounds: a scene builds its own on the device, which are shorter (so a
+ * grid reported as dropped past the entry cap may be kept there), and hard
+ * unions have grids that are not reported here. */
 typedef struct ft_build_info {
   uint32_t leaves;
   uint32_t primitive_leaves;
